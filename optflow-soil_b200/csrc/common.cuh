@@ -56,19 +56,46 @@ inline unsigned div_up(size_t a, size_t b) { return (unsigned)((a + b - 1) / b);
 // (the pair driver's lanes) must not shrink it under each other's launches
 void raise_smem_limit(const void* fn, size_t bytes);
 
+// two float32 values in a 64-bit register pair; fma on both halves in one instruction, each rounded as fmaf
+__device__ __forceinline__ unsigned long long f32x2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f32x2_split(unsigned long long v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // atan2(y, x) in float32 for finite or NaN arguments, from the mathematics: with a = min(|x|, |y|) / max(|x|, |y|)
 // in [0, 1], atan(a) = a P(a^2), P the 8-term fit of atan(a) / a made by atan_fit.py (a minimax fit of the relative
 // error by iteratively reweighted least squares; 1.6e-7 rad at most in a float32 Horner); then pi/2 - r where
 // |y| > |x|, pi - r where x is negative (its sign bit: -0 included) and the sign of y (+-0 as atan2 gives them).
 // At most 5e-7 rad (about 2 ulp of pi) from the exact angle of the float32 arguments with the quotient's rounding and
-// the reflections; NaN in gives NaN; atan2(+-0, +0) = +-0 and atan2(+-0, -0) = +-pi.
-__device__ __forceinline__ float atan2_phase(float y, float x) {
-  if (y != y || x != x) return y + x;
-  const float ax = fabsf(x), ay = fabsf(y);
+// the reflections; NaN in gives NaN; atan2(+-0, +0) = +-0 and atan2(+-0, -0) = +-pi. The quotient is the fast one in
+// the reciprocal's range; magnitudes outside [1e-30, 1e30] are scaled into it by a power of two (a select, no branch).
+__device__ __forceinline__ float atan2_ratio(float ax, float ay) {
   const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
-  float a;
-  if (mx > 1e-30f && mx < 1e30f) a = __fdividef(mn, mx);  // the reciprocal's range: a fast quotient
-  else a = mx > 0.f ? mn / mx : 0.f;
+  const float sc = mx < 1e-30f ? 0x1p96f : (mx > 1e30f ? 0x1p-96f : 1.f);
+  return __fdividef(mn * sc, fmaxf(mx * sc, 1e-30f));  // 0 / 0 becomes 0
+}
+// r = atan(min / max) reflected into the argument's octant
+__device__ __forceinline__ float atan2_octant(float r, float x, float y) {
+  if (fabsf(y) > fabsf(x)) r = 1.57079632679489662f - r;
+  if (signbit(x)) r = 3.14159265358979324f - r;
+  return copysignf(r, y);
+}
+__device__ __forceinline__ float atan2_phase(float y, float x) {
+  const float a = atan2_ratio(fabsf(x), fabsf(y));
   const float t = a * a;
   float p = -4.693272372e-03f;
   p = fmaf(p, t, 2.425239656e-02f);
@@ -78,10 +105,25 @@ __device__ __forceinline__ float atan2_phase(float y, float x) {
   p = fmaf(p, t, 1.996972415e-01f);
   p = fmaf(p, t, -3.333199078e-01f);
   p = fmaf(p, t, 9.999999010e-01f);
-  float r = p * a;
-  if (ay > ax) r = 1.57079632679489662f - r;
-  if (signbit(x)) r = 3.14159265358979324f - r;
-  return copysignf(r, y);
+  const float r = atan2_octant(p * a, x, y);
+  return (y != y || x != x) ? y + x : r;
+}
+// atan2_phase of two arguments with the polynomial of both in packed instructions: the same value for numbers. A NaN
+// argument may give any angle: the caller's weight |r1| |r2| is NaN then, and with it every sum
+__device__ __forceinline__ void atan2_phase_pair(float y0, float x0, float y1, float x1, float& r0, float& r1) {
+  const unsigned long long a = f32x2(atan2_ratio(fabsf(x0), fabsf(y0)), atan2_ratio(fabsf(x1), fabsf(y1)));
+  const unsigned long long t = mul_f32x2(a, a);
+  unsigned long long p = f32x2(-4.693272372e-03f, -4.693272372e-03f);
+  p = fma_f32x2(p, t, f32x2(2.425239656e-02f, 2.425239656e-02f));
+  p = fma_f32x2(p, t, f32x2(-5.948639446e-02f, -5.948639446e-02f));
+  p = fma_f32x2(p, t, f32x2(9.914293821e-02f, 9.914293821e-02f));
+  p = fma_f32x2(p, t, f32x2(-1.401948170e-01f, -1.401948170e-01f));
+  p = fma_f32x2(p, t, f32x2(1.996972415e-01f, 1.996972415e-01f));
+  p = fma_f32x2(p, t, f32x2(-3.333199078e-01f, -3.333199078e-01f));
+  p = fma_f32x2(p, t, f32x2(9.999999010e-01f, 9.999999010e-01f));
+  f32x2_split(mul_f32x2(p, a), r0, r1);
+  r0 = atan2_octant(r0, x0, y0);
+  r1 = atan2_octant(r1, x1, y1);
 }
 
 // ---------------------------------------------------------------- cubic B-spline (interp.py)

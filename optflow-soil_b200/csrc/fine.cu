@@ -348,141 +348,218 @@ void launch_warp_gather(const float* c2, int w2, int h2, const double* sx, const
 // One pixel per thread. The fixed point X' + s(X') = X + u(X) and the positions are float64; the responses are
 // sampled with float32 weights and accumulation (they are stored as complex float32), and the phase difference
 // angle(r1 conj(r2)) is taken in float32 by atan2_phase (the inputs carry float32 precision; the angle is within
-// 5e-7 rad of theirs, at about half the instructions of atan2f); c = dphi + gx u + gy v and the seven sums are float64, since u reaches tens of pixels and the residual
-// sum gcc - theta . b cancels. The kernel is latency-bound, so: the F reference-pack values of the pixel are
-// copied to shared memory asynchronously at the start (in flight during the fixed point); |r1| |r2| is one square
-// root of |r1|^2 |r2|^2, with |r1|^2 formed from the pack; the 16 tap offsets are computed once and reused by every
-// filter; the field spline is stored interleaved (one 16-byte load per tap for both components); the responses are
+// 5e-7 rad of theirs); c = dphi + gx u + gy v and the seven sums are float64, since u reaches tens of pixels and the
+// residual sum gcc - theta . b cancels. |r1| |r2| is one square root of |r1|^2 |r2|^2, with |r1|^2 formed from the
+// pack; the field spline is stored interleaved (one 16-byte load per tap for both components); the responses are
 // stored in filter pairs, node-major, so one 16-byte load per tap serves two filters (96 tap loads per pixel at F = 12
 // instead of 192).
-constexpr int ACC_BX = 32, ACC_BY = 8, ACC_T = ACC_BX * ACC_BY;
-#ifndef ACC_MINB
-#define ACC_MINB 4
-#endif
-__global__ void __launch_bounds__(ACC_T, ACC_MINB) k_accumulate(const float4* __restrict__ ref4, const float2* __restrict__ R,
+// What bounds it is the latency and the issue slots of about 2200 instructions per pixel (DRAM at a third). Measured at
+// 2048^2, F = 12, against 0.572 ms per launch before (the same sums bit for bit):
+//   - the reference pack comes by asynchronous copies into a ring of two filter pairs instead of all F filters at once:
+//     32 KB of shared memory per SM instead of 192 KB leave L1 room for the taps of the resident blocks (0.573 ->
+//     0.534 ms with the changes below; a ring of three pairs 0.482 against 0.478 ms);
+//   - the taps' float32 sums and the two filters' atan polynomials run in packed instructions (fma.rn.f32x2: two
+//     values per issue slot, each rounded as by fmaf), the quotient of atan2 needs no branch, and the positions whose
+//     taps would mirror or clamp (at the plane's border) go out of line, so that the rest tests its range once;
+//   - 32 x 4 pixels per block, 7 blocks per SM at 72 registers: 0.478 ms (8 blocks at 64 registers 0.503, 6 at 80
+//     0.507, 32 x 8 pixels at 4 blocks 0.503).
+// Slower, and not kept: two pixels of a column per thread sharing their tap rows (L1 wavefronts fall by a third, but
+// 128 registers leave 16 warps per SM: 0.66 ms); the fixed point in a kernel of its own (0.122 + 0.424 ms: its loads no
+// longer overlap the sums' arithmetic).
+constexpr int ACC_BX = 32, ACC_BY = 4, ACC_T = ACC_BX * ACC_BY, ACC_MINB = 7;
+constexpr int ACC_ST = 2;       // filter pairs in the ring of the reference pack
+constexpr int ACC_MAXF = 56;    // the filters an earlier form held in shared memory at once; more stay refused
+
+// the taps of a position at least one node inside the plane in both directions (no clamp, no reflection: what make_taps
+// gives there); false elsewhere and for NaN
+__device__ __forceinline__ bool taps_inside(double x, double y, int w, int h, int& node, double (&wx)[4], double (&wy)[4]) {
+  if (!(x >= 1.0 && x < (double)(w - 2) && y >= 1.0 && y < (double)(h - 2))) return false;
+  const double fx = floor(x), fy = floor(y);
+  node = ((int)fy - 1) * w + ((int)fx - 1);
+  bspline_weights(x - fx, wx);
+  bspline_weights(y - fy, wy);
+  return true;
+}
+
+// the field spline at (x, y) by the general taps
+__device__ __noinline__ double2 field_general(const double2* __restrict__ cs, int W, int H, double x, double y) {
+  Taps t;
+  if (!make_taps(x, y, W, H, t)) return make_double2(nan(""), nan(""));
+  return sample_pair(cs, W, t);
+}
+
+// the contributions of filters of phase difference dphi to a pixel's seven sums, from a filter's pack r1 (re, im, gx, gy)
+// and its complex response sample b at X' (r2 of phaseflow.py:476-483)
+__device__ __forceinline__ void acc_add(double (&a)[7], float4 r1, float br, float bi, float dph, double u, double v) {
+  // |r1|^2 as the reference pack's amplitude squared (phaseflow.py:111), from the stored float32 response
+  const float q1 = fmaf(r1.x, r1.x, fmaf(r1.y, r1.y, 1e-12f));
+  const double dphi = (double)dph;
+  const double wk = (double)sqrtf(q1 * fmaf(br, br, bi * bi));  // |r1| |r2|
+  const double gx = r1.z, gy = r1.w;
+  const double c = dphi + gx * u + gy * v;
+  const double wgx = wk * gx, wgy = wk * gy;
+  a[0] = fma(wgx, gx, a[0]);
+  a[1] = fma(wgx, gy, a[1]);
+  a[2] = fma(wgy, gy, a[2]);
+  a[3] = fma(wgx, c, a[3]);
+  a[4] = fma(wgy, c, a[4]);
+  a[5] = fma(wk * c, c, a[5]);
+  a[6] += wk;
+}
+// r1 conj(r2)
+__device__ __forceinline__ void acc_cross(float4 r1, float br, float bi, float& im, float& re) {
+  re = fmaf(r1.x, br, r1.y * bi);
+  im = fmaf(r1.y, br, -r1.x * bi);
+}
+
+// a pixel whose taps mirror at the padded plane's border, or whose position is NaN: the general taps, from the pack in
+// global memory
+__device__ __noinline__ void acc_general(const float4* __restrict__ ref4, const float4* __restrict__ R4, int F, int ph,
+                                         int pw, size_t N, size_t p, double px, double py, double u, double v,
+                                         double* __restrict__ sums) {
+  const float fnan = __int_as_float(0x7fc00000);
+  const size_t plane = (size_t)ph * pw;
+  double a[7] = {0, 0, 0, 0, 0, 0, 0};
+  Taps t;
+  const bool ok = make_taps(px + PAD, py + PAD, pw, ph, t);
+#pragma unroll 1
+  for (int k = 0; k < F; k++) {
+    float br = fnan, bi = fnan;
+    if (ok) {
+      br = bi = 0.f;
+      const float2* Rk = (const float2*)(R4 + (size_t)(k >> 1) * plane) + (k & 1);
+#pragma unroll 1
+      for (int jj = 0; jj < 4; jj++) {
+        float ar = 0.f, ai = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const float2 cv = __ldg(Rk + 2 * ((size_t)t.yi[jj] * pw + t.xi[q]));
+          ar = fmaf((float)t.wx[q], cv.x, ar);
+          ai = fmaf((float)t.wx[q], cv.y, ai);
+        }
+        br = fmaf((float)t.wy[jj], ar, br);
+        bi = fmaf((float)t.wy[jj], ai, bi);
+      }
+    }
+    const float4 r1 = __ldg(ref4 + (size_t)k * N + p);
+    float im, re;
+    acc_cross(r1, br, bi, im, re);
+    acc_add(a, r1, br, bi, atan2_phase(im, re), u, v);
+  }
+#pragma unroll
+  for (int i = 0; i < 7; i++) sums[i * N + p] = a[i];
+}
+
+__global__ void __launch_bounds__(ACC_T, ACC_MINB) k_accumulate(const float4* __restrict__ ref4, const float4* __restrict__ R4,
                                                       int F, int ph, int pw, const double* __restrict__ ux,
                                                       const double* __restrict__ uy, const double* __restrict__ sx,
                                                       const double* __restrict__ sy, const double2* __restrict__ cs,
                                                       int W, int H, double* __restrict__ sums) {
-  extern __shared__ float4 pk[];  // F x ACC_T
+  extern __shared__ float4 pk[];  // ACC_ST x 2 x ACC_T
   // a block covers ACC_BX x ACC_BY pixels: its warps' response taps share rows in L1
   const int x = blockIdx.x * ACC_BX + threadIdx.x, y = blockIdx.y * ACC_BY + threadIdx.y;
   const int tid = threadIdx.y * ACC_BX + threadIdx.x;
   if (x >= W || y >= H) return;
   const size_t N = (size_t)W * H;
   const size_t p = (size_t)y * W + x;
-  for (int k = 0; k < F; k++) __pipeline_memcpy_async(&pk[k * ACC_T + tid], ref4 + (size_t)k * N + p, 16);
-  __pipeline_commit();
+  // the reference pack of filter pair j into its slot of the ring (one group of asynchronous copies; an empty group
+  // past the end)
+  auto fetch = [&](int j) {
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+      if (2 * j + c < F)
+        __pipeline_memcpy_async(&pk[((j % ACC_ST) * 2 + c) * ACC_T + tid], ref4 + (size_t)(2 * j + c) * N + p, 16);
+    __pipeline_commit();
+  };
+#pragma unroll
+  for (int j = 0; j < ACC_ST - 1; j++) fetch(j);
   const double u = ux[p], v = uy[p];
   const double tx = x + u, ty = y + v;
   double px = tx - sx[p], py = ty - sy[p];
+  int base;
+  double dwx[4], dwy[4];
   // X' + s(X') = X + u(X): two fixed-point steps on the spline of s (phaseflow.py:469-472)
+#pragma unroll 1
   for (int it = 0; it < 2; it++) {
-    Taps t;
-    double nx, ny;
-    if (make_taps(px, py, W, H, t)) {
-      const double2 sv = sample_pair(cs, W, t);
-      nx = tx - sv.x;
-      ny = ty - sv.y;
+    double o1 = 0, o2 = 0;
+    if (taps_inside(px, py, W, H, base, dwx, dwy)) {
+      const double2* row = cs + base;
+#pragma unroll
+      for (int j = 0; j < 4; j++, row += W) {
+        const double2 c0 = __ldg(row);
+        double a1 = dwx[0] * c0.x, a2 = dwx[0] * c0.y;
+#pragma unroll
+        for (int k = 1; k < 4; k++) {
+          const double2 cv = __ldg(row + k);
+          a1 += dwx[k] * cv.x;
+          a2 += dwx[k] * cv.y;
+        }
+        o1 += dwy[j] * a1;
+        o2 += dwy[j] * a2;
+      }
     } else {
-      nx = ny = nan("");
+      const double2 sv = field_general(cs, W, H, px, py);
+      o1 = sv.x;
+      o2 = sv.y;
     }
-    px = nx;
-    py = ny;
+    px = tx - o1;
+    py = ty - o2;
   }
-  double a0 = 0, a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0, a6 = 0;
-  Taps t;
-  const bool ok = make_taps(px + PAD, py + PAD, pw, ph, t);
-  float fwx[4], fwy[4];
+  if (!taps_inside(px + PAD, py + PAD, pw, ph, base, dwx, dwy)) {
+    __pipeline_wait_prior(0);
+    acc_general(ref4, R4, F, ph, pw, N, p, px, py, u, v, sums);
+    return;
+  }
+  unsigned long long wx[4], wy[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    fwx[k] = (float)t.wx[k];
-    fwy[k] = (float)t.wy[k];
+    const float a = (float)dwx[k], b = (float)dwy[k];
+    wx[k] = f32x2(a, a);
+    wy[k] = f32x2(b, b);
   }
+  double a[7] = {0, 0, 0, 0, 0, 0, 0};
   const size_t plane = (size_t)ph * pw;
-  const float fnan = __int_as_float(0x7fc00000);
-  // filter k's contribution from its complex response sample b at X' (r2 of phaseflow.py:476-483)
-  auto add = [&](int k, float br, float bi) {
-    const float4 r1 = pk[k * ACC_T + tid];
-    // |r1|^2 as the reference pack's amplitude squared (phaseflow.py:111), from the stored float32 response
-    const float q1 = fmaf(r1.x, r1.x, fmaf(r1.y, r1.y, 1e-12f));
-    // r1 conj(r2)
-    const float re = fmaf(r1.x, br, r1.y * bi);
-    const float im = fmaf(r1.y, br, -r1.x * bi);
-    const double dphi = (double)atan2_phase(im, re);
-    const double wk = (double)sqrtf(q1 * fmaf(br, br, bi * bi));  // |r1| |r2|
-    const double gx = r1.z, gy = r1.w;
-    const double c = dphi + gx * u + gy * v;
-    const double wgx = wk * gx, wgy = wk * gy;
-    a0 = fma(wgx, gx, a0);
-    a1 = fma(wgx, gy, a1);
-    a2 = fma(wgy, gy, a2);
-    a3 = fma(wgx, c, a3);
-    a4 = fma(wgy, c, a4);
-    a5 = fma(wk * c, c, a5);
-    a6 += wk;
-  };
-  // the responses in filter pairs, node-major: one 16-byte load per tap gives both filters of a pair. A pair's
-  // sample from its plane Rj, tap (jj, q) at Rj + off(jj, q); the next pair's tap rows go into L1 meanwhile
-  const float4* R4 = reinterpret_cast<const float4*>(R);
+  // the responses in filter pairs, node-major: one 16-byte load per tap gives both filters of a pair; the taps are a
+  // block (one address per row, the four loads at fixed offsets from it)
+  const ulonglong2* Rj = reinterpret_cast<const ulonglong2*>(R4) + base;
   const int npairs = (F + 1) >> 1;
-  auto pair_sample = [&](const float4* Rj, bool next, auto off, float& b0r, float& b0i, float& b1r, float& b1i) {
-    if (next) {
+#pragma unroll 1
+  for (int j = 0; j < npairs; j++, Rj += plane) {
+    // the next pair's tap rows go into L1 meanwhile
+    if (j + 1 < npairs) {
 #pragma unroll
-      for (int jj = 0; jj < 4; jj++) asm volatile("prefetch.global.L1 [%0];" ::"l"(Rj + plane + off(jj, 0)));
+      for (int r = 0; r < 4; r++) asm volatile("prefetch.global.L1 [%0];" ::"l"(Rj + plane + r * pw));
     }
-    b0r = b0i = b1r = b1i = 0.f;
+    unsigned long long s0 = 0ull, s1 = 0ull;
 #pragma unroll
-    for (int jj = 0; jj < 4; jj++) {
-      float a0r = 0.f, a0i = 0.f, a1r = 0.f, a1i = 0.f;
+    for (int r = 0; r < 4; r++) {
+      unsigned long long r0 = 0ull, r1 = 0ull;
 #pragma unroll
       for (int q = 0; q < 4; q++) {
-        const float4 cv = __ldg(Rj + off(jj, q));
-        a0r = fmaf(fwx[q], cv.x, a0r);
-        a0i = fmaf(fwx[q], cv.y, a0i);
-        a1r = fmaf(fwx[q], cv.z, a1r);
-        a1i = fmaf(fwx[q], cv.w, a1i);
+        const ulonglong2 c = __ldg(Rj + (r * pw + q));
+        r0 = fma_f32x2(wx[q], c.x, r0);
+        r1 = fma_f32x2(wx[q], c.y, r1);
       }
-      b0r = fmaf(fwy[jj], a0r, b0r);
-      b0i = fmaf(fwy[jj], a0i, b0i);
-      b1r = fmaf(fwy[jj], a1r, b1r);
-      b1i = fmaf(fwy[jj], a1i, b1i);
+      s0 = fma_f32x2(wy[r], r0, s0);
+      s1 = fma_f32x2(wy[r], r1, s1);
     }
-  };
-  __pipeline_wait_prior(0);
-  if (ok && t.cx && t.yi[1] == t.yi[0] + 1 && t.yi[2] == t.yi[0] + 2 && t.yi[3] == t.yi[0] + 3) {
-    // no reflection in either direction (all but the positions within a node of the padded plane's edge): the 4 x 4
-    // taps are a block, one address per row and the four loads at fixed offsets from it
-    const float4* Rj = R4 + ((size_t)t.yi[0] * pw + t.xi[0]);
-    for (int j = 0; j < npairs; j++, Rj += plane) {
-      float b0r, b0i, b1r, b1i;
-      pair_sample(Rj, j + 1 < npairs, [&](int jj, int q) { return jj * pw + q; }, b0r, b0i, b1r, b1i);
-      add(2 * j, b0r, b0i);
-      if (2 * j + 1 < F) add(2 * j + 1, b1r, b1i);
-    }
-  } else {
-    int ro[4], xo[4];  // tap (j, q) at ro[j] + xo[q] in a filter's plane
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      ro[k] = ok ? t.yi[k] * pw : 0;
-      xo[k] = ok ? t.xi[k] : 0;
-    }
-    for (int j = 0; j < npairs; j++) {
-      float b0r = fnan, b0i = fnan, b1r = fnan, b1i = fnan;
-      if (ok)
-        pair_sample(R4 + (size_t)j * plane, j + 1 < npairs, [&](int jj, int q) { return ro[jj] + xo[q]; }, b0r, b0i,
-                    b1r, b1i);
-      add(2 * j, b0r, b0i);
-      if (2 * j + 1 < F) add(2 * j + 1, b1r, b1i);
-    }
+    fetch(j + ACC_ST - 1);
+    __pipeline_wait_prior(ACC_ST - 1);
+    float b0r, b0i, b1r, b1i;
+    f32x2_split(s0, b0r, b0i);
+    f32x2_split(s1, b1r, b1i);
+    const float4* slot = pk + (j % ACC_ST) * 2 * ACC_T + tid;
+    const float4 ra = slot[0], rb = slot[ACC_T];  // rb: stale for the odd filter's copy, unused then
+    float im0, re0, im1, re1, d0, d1;
+    acc_cross(ra, b0r, b0i, im0, re0);
+    acc_cross(rb, b1r, b1i, im1, re1);
+    atan2_phase_pair(im0, re0, im1, re1, d0, d1);
+    acc_add(a, ra, b0r, b0i, d0, u, v);
+    if (2 * j + 1 < F) acc_add(a, rb, b1r, b1i, d1, u, v);
   }
-  sums[p] = a0;
-  sums[N + p] = a1;
-  sums[2 * N + p] = a2;
-  sums[3 * N + p] = a3;
-  sums[4 * N + p] = a4;
-  sums[5 * N + p] = a5;
-  sums[6 * N + p] = a6;
+  __pipeline_wait_prior(0);
+#pragma unroll
+  for (int i = 0; i < 7; i++) sums[i * N + p] = a[i];
 }
 
 // the accumulate as a gather from the response planes: the form for planes without tensor maps, and the reference
@@ -491,10 +568,11 @@ void launch_accumulate_gather(const float4* ref4, const float2* R, int F, int ph
                               const double* uy, const double* sx, const double* sy, const double2* cs, int W, int H,
                               double* sums, cudaStream_t st) {
   dim3 g(div_up(W, ACC_BX), div_up(H, ACC_BY));
-  const size_t sm = (size_t)F * ACC_T * sizeof(float4);
-  if (sm > 227 * 1024) throw Error(OFC_ERR_WINDOW, "too many Gabor filters (" + std::to_string(F) + ") for the CUDA engine");
+  const size_t sm = (size_t)2 * ACC_ST * ACC_T * sizeof(float4);
+  if (F > ACC_MAXF)
+    throw Error(OFC_ERR_WINDOW, "too many Gabor filters (" + std::to_string(F) + ") for the CUDA engine");
   raise_smem_limit((const void*)k_accumulate, sm);
-  OFC_LAUNCH(k_accumulate, g, dim3(ACC_BX, ACC_BY), sm, st, ref4, R, F, ph, pw, ux, uy, sx, sy, cs, W, H, sums);
+  OFC_LAUNCH(k_accumulate, g, dim3(ACC_BX, ACC_BY), sm, st, ref4, (const float4*)R, F, ph, pw, ux, uy, sx, sy, cs, W, H, sums);
 }
 
 // ---------------------------------------------------------------- window moments + solve

@@ -251,6 +251,28 @@ def test_accumulate_tma_matches_gather(T, shape, amp):
     np.testing.assert_array_equal(s1, s0)
 
 
+@pytest.mark.parametrize("shape,n_orient,scales", [((64, 65), 1, (1.0,)), ((67, 131), 3, (0.6,)), ((130, 97), 5, (0.6,)),
+                                                   ((70, 64), 4, (0.6, 1.0, 1.6))])
+def test_accumulate_ring_and_edges(T, shape, n_orient, scales):
+    """The gather accumulate (the reference pack in a ring of two filter pairs, packed sampling, border positions out of
+    line) against the TMA-staged kernel's unpacked arithmetic bit for bit: one filter, odd filter counts (the last pair
+    half empty), sizes off the 32 x 4 block, positions beyond the padded plane on every side."""
+    rng = np.random.default_rng(shape[1])
+    h, w = shape
+    a, b = rng.random((h, w)), rng.random((h, w))
+    yy, xx = np.mgrid[0:h, 0:w].astype(np.float64)
+    ux, uy = 3 * np.sin(xx / 17.0), 2 * np.cos(yy / 23.0)
+    ux[:, :4] -= 70.0
+    ux[:, -4:] += 70.0
+    uy[:5] -= 70.0
+    uy[-5:] += 70.0
+    cfg = Config(n_orient=n_orient, scales=scales)
+    s0, _ = T.accumulate(a, b, ux, uy, mode=0, cfg=cfg)
+    s1, t1 = T.accumulate(a, b, ux, uy, mode=1, cfg=cfg)
+    assert t1 == 0 and np.isfinite(s1).all()
+    np.testing.assert_array_equal(s0, s1)
+
+
 def test_atan2_phase(T):
     """The accumulate's float32 atan2 (common.cuh, a polynomial fit of atan on [0, 1]) within 5e-7 rad of the exact
     angle of its float32 arguments over 20 decades of magnitude and every direction, like CUDA's atan2f there; signed
