@@ -2,6 +2,7 @@
 // rust/crates/optflow-core/src/phaseflow.rs:1514-1613): smoothing, splines, warp, accumulate, window moments
 // and the local solve, the energy median, the confidence and the trusted pre-warp.
 #include <cfloat>
+#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -789,104 +790,126 @@ __global__ void __launch_bounds__(128) k_moments_x_solve(const double* __restric
   }
 }
 
-// ---- register-blocked window moments for the default window (r = MOM_R = 16, 33 taps)
-// y pass: a thread owns RY consecutive rows of one column; it loads the RY + 2r rows of a source plane once
-// (instead of 2r + 1 loads per output row, most of them L2 traffic) and forms every y-plane of that source,
-// with the tap loop outermost so that the RY x (powers) accumulators advance side by side (independent
-// float64 chains: the pass is bound by float64 latency otherwise).
-constexpr int MOM_RY = 4;
-
-template <int ORDER>
-__global__ void __launch_bounds__(128, 4) k_moments_y_rb(const double* __restrict__ sums, int W, int H, MomTaps tp,
-                                                         double* __restrict__ yplanes) {
-  constexpr MomTable T = build_table(ORDER);
-  constexpr int R = MOM_R, RY = MOM_RY, NV = RY + 2 * R;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y0 = blockIdx.y * RY;
-  if (x >= W) return;
-  const size_t N = (size_t)W * H;
+// ---- window moments for the default window (r = MOM_R = 16, 33 taps) through shared memory
+// Both passes walk the tap pairs outward from a thread's RB consecutive outputs with two sliding register windows
+// (the RB samples at +t and the RB at -t; a step of t shifts each by one and loads one sample), so RB outputs take
+// RB + 32 shared-memory loads and 2 RB + RB x powers live values.
+// outputs j of powers 0 .. NP - 1 from the samples v(i), i = 0 .. RB + 31 (output j's centre at i = j + 16)
+template <int RB, int NP, class V>
+__device__ __forceinline__ void mom_slide(V v, const MomTaps& tp, double (&acc)[RB][NP]) {
+  constexpr int R = MOM_R;
+  double up[RB], dn[RB];
 #pragma unroll
-  for (int src = 0; src < 7; src++) {
-    bool used = false;
-    bool pw[5] = {false, false, false, false, false};
+  for (int j = 0; j < RB; j++) {
 #pragma unroll
-    for (int j = 0; j < T.ny; j++)
-      if (T.ysrc[j] == src) {
-        used = true;
-        pw[T.ypow[j]] = true;
-      }
-    if (!used) continue;
-    const double* plane = sums + (size_t)src * N + x;
-    double v[NV];
+    for (int p = 0; p < NP; p++) acc[j][p] = p == 0 ? tp.k[0][0] * v(j + R) : 0.0;
+    up[j] = v(j + R + 1);
+    dn[j] = v(j + R - 1);
+  }
 #pragma unroll
-    for (int i = 0; i < NV; i++) v[i] = plane[(size_t)min(max(y0 - R + i, 0), H - 1) * W];
-    double acc[RY][5];
+  for (int t = 1; t <= R; t++) {
 #pragma unroll
-    for (int j = 0; j < RY; j++)
+    for (int j = 0; j < RB; j++) {
+      const double sp = up[j] + dn[j], dm = up[j] - dn[j];
 #pragma unroll
-      for (int p = 0; p < 5; p++) acc[j][p] = p == 0 ? tp.k[0][0] * v[j + R] : 0.0;
+      for (int p = 0; p < NP; p++) acc[j][p] = fma(tp.k[p][t], (p & 1) ? dm : sp, acc[j][p]);
+    }
+    if (t < R) {
 #pragma unroll
-    for (int t = 1; t <= R; t++)
+      for (int j = 0; j + 1 < RB; j++) up[j] = up[j + 1];
+      up[RB - 1] = v(R + t + RB);
 #pragma unroll
-      for (int j = 0; j < RY; j++) {
-        const double sp = v[j + R + t] + v[j + R - t], dm = v[j + R + t] - v[j + R - t];
-#pragma unroll
-        for (int p = 0; p < 5; p++)
-          if (pw[p]) acc[j][p] = fma(tp.k[p][t], (p & 1) ? dm : sp, acc[j][p]);
-      }
-#pragma unroll
-    for (int j = 0; j < RY; j++) {
-      if (y0 + j >= H) break;
-      const size_t o = (size_t)(y0 + j) * W + x;
-#pragma unroll
-      for (int q = 0; q < T.ny; q++)
-        if (T.ysrc[q] == src) yplanes[(size_t)q * N + o] = acc[j][T.ypow[q]];
+      for (int j = RB - 1; j > 0; j--) dn[j] = dn[j - 1];
+      dn[0] = v(R - t - 1);
     }
   }
 }
 
-// x pass + solve: a block owns a row segment of SEG = GT RX pixels and has two groups of GT threads. The groups
-// take the y-planes in pairs, group g plane Q + g of each pair: a group stages its plane's segment and 2r halo in
-// shared memory (double-buffered per group, its next plane's loads in flight meanwhile); a thread takes the RX + 2r
-// values around its RX consecutive pixels into registers (an odd RX keeps the warp's reads on distinct banks) and
-// writes their moments into a shared tile of nm x SEG (tap loop outermost, RX x powers accumulators side by side).
-// Then every thread of the block solves the pixels tid, tid + 2 GT, ... from the tile. Two groups give twice the warps
-// per SM of one group of GT threads at the same tile (the tile, 8 nm bytes per pixel, bounds the blocks per SM), and
-// each moment is formed by the same operations in the same order either way. Order 1 runs 4 blocks per SM (110
-// registers); order 2 runs 2 (its 12 x 12 solve in registers takes 218).
+// the y-planes of a source: the number of y powers it feeds (a prefix 0 .. np - 1) and the plane of each
+struct SrcPlanes {
+  int np[7] = {};
+  int plane[7][5] = {};
+};
+__host__ __device__ constexpr SrcPlanes build_src_planes(int order) {
+  SrcPlanes r{};
+  const MomTable T = build_table(order);
+  for (int q = 0; q < T.ny; q++) {
+    r.plane[T.ysrc[q]][T.ypow[q]] = q;
+    if (T.ypow[q] + 1 > r.np[T.ysrc[q]]) r.np[T.ysrc[q]] = T.ypow[q] + 1;
+  }
+  return r;
+}
+__constant__ SrcPlanes c_src_planes[2] = {build_src_planes(1), build_src_planes(2)};
+
+// y pass: a block takes 32 columns x 8 RY rows of one source plane (blockIdx.z) and its 2r halo rows into shared memory
+// (asynchronous copies), a warp RY rows of them. Bound by the float64 pipe (63 % busy) and its 15 output planes; the loads
+// of a tile wait behind other blocks' arithmetic. Order 1 at 2048^2: 0.162 ms with 6 rows per warp lane and 3 blocks of 256
+// threads per SM (78 registers) against 0.208 ms for 36 global loads per 4 outputs; 4 rows 0.169, 8 rows (128 registers)
+// 0.189. Order 2 (up to 5 powers) keeps 4 rows: 64 registers without spills.
+constexpr int MY_W = 8;
+template <int ORDER>
+struct MomY {
+  static constexpr int RY = ORDER == 1 ? 6 : 4, MINB = ORDER == 1 ? 3 : 4;
+};
+template <int ORDER>
+__global__ void __launch_bounds__(32 * MY_W, MomY<ORDER>::MINB) k_moments_y_rb(const double* __restrict__ sums, int W, int H, MomTaps tp,
+                                                             double* __restrict__ yplanes) {
+  constexpr int R = MOM_R, RY = MomY<ORDER>::RY, TB = MY_W * RY, NR = TB + 2 * R;
+  static_assert(NR % MY_W == 0, "whole rows of the tile per warp");
+  __shared__ double tile[NR * 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, src = blockIdx.z;
+  const int x = blockIdx.x * 32 + lane, y0 = blockIdx.y * TB;
+  const size_t N = (size_t)W * H;
+  const double* plane = sums + (size_t)src * N + x;
+  if (x < W) {
+#pragma unroll
+    for (int i = 0; i < NR / MY_W; i++) {
+      const int r = wid + MY_W * i;
+      __pipeline_memcpy_async(tile + r * 32 + lane, plane + (size_t)min(max(y0 - R + r, 0), H - 1) * W, sizeof(double));
+    }
+  }
+  __pipeline_commit();
+  __pipeline_wait_prior(0);
+  __syncthreads();
+  const int yb = y0 + wid * RY;
+  if (x >= W || yb >= H) return;
+  const double* t0 = tile + wid * RY * 32 + lane;
+  const SrcPlanes& SP = c_src_planes[ORDER - 1];
+  auto run = [&](auto npc) {
+    constexpr int NP = decltype(npc)::value;
+    double acc[RY][NP];
+    mom_slide<RY, NP>([&](int i) { return t0[i * 32]; }, tp, acc);
+#pragma unroll
+    for (int p = 0; p < NP; p++) {
+      double* o = yplanes + (size_t)SP.plane[src][p] * N + (size_t)yb * W + x;
+#pragma unroll
+      for (int j = 0; j < RY; j++) {
+        if (yb + j < H) o[(size_t)j * W] = acc[j][p];
+      }
+    }
+  };
+  const int np = SP.np[src];  // order 1: 3 (products), 2 (right sides), 1; order 2: 5, 3, 1
+  if (np == 1) run(std::integral_constant<int, 1>{});
+  else if (np == 3) run(std::integral_constant<int, 3>{});
+  else if (ORDER == 1) run(std::integral_constant<int, 2>{});
+  else run(std::integral_constant<int, 5>{});
+}
+
+// x pass + solve: a block owns a row segment of SEG = 32 RX pixels and has G warps that share out its y-planes (a fixed
+// balanced schedule). A warp stages its plane's segment and 2r halo in a buffer of its own (double-buffered asynchronous
+// copies; only warp barriers), a lane forms the moments of RX consecutive pixels (an odd RX keeps the lanes' reads on
+// distinct banks) and writes them into a shared tile of nm x SEG. Then the block's threads solve a pixel each from the
+// tile. The float64 pipe bounds it (69 % busy; the solve is a third of its work), and a lane's sample loads next:
+// (RX + 32) / RX per pixel and plane. Order 1 at 2048^2: 0.334 ms with 5 pixels per lane, 4 warps, 4 blocks per SM (117
+// registers) against 0.393 ms for two groups of 64 threads with 3 pixels each; 3 pixels 0.36-0.38, 7 pixels 0.395, 5
+// warps at 96 registers 0.335. Order 2 (59 moments per pixel bound the tile, the 12 x 12 solve the registers) at 512^2:
+// 88 us with 3 pixels per lane against 131 us with one.
 template <int ORDER>
 struct MomX {
-  static constexpr int RX = ORDER == 1 ? 3 : 1;
-  static constexpr int GT = 64, NT = 2 * GT, SEG = GT * RX, WIN = SEG + 2 * MOM_R;
-  static constexpr size_t smem() { return (size_t)(4 * WIN + build_table(ORDER).nm * SEG) * sizeof(double); }
+  static constexpr int RX = ORDER == 1 ? 5 : 3, G = 4, MINB = ORDER == 1 ? 4 : 2;
+  static constexpr int NT = 32 * G, SEG = 32 * RX, WIN = SEG + 2 * MOM_R;
+  static constexpr size_t smem() { return (size_t)(2 * G * WIN + build_table(ORDER).nm * SEG) * sizeof(double); }
 };
-
-// the NPF values of a row segment (with its halo) that thread lt of a group stages: i = lt + GT j
-template <int ORDER>
-struct MomPf {
-  static constexpr int NPF = (MomX<ORDER>::WIN + MomX<ORDER>::GT - 1) / MomX<ORDER>::GT;
-  double v[NPF];
-};
-
-template <int ORDER>
-__device__ __forceinline__ void mom_x_fetch(const double* __restrict__ row, int x0, int W, int lt, MomPf<ORDER>& pf) {
-  constexpr int R = MOM_R, GT = MomX<ORDER>::GT, WIN = MomX<ORDER>::WIN;
-#pragma unroll
-  for (int j = 0; j < MomPf<ORDER>::NPF; j++) {
-    const int i = lt + GT * j;
-    if (i < WIN) pf.v[j] = row[min(max(x0 - R + i, 0), W - 1)];
-  }
-}
-
-template <int ORDER>
-__device__ __forceinline__ void mom_x_stage(double* wb, int lt, const MomPf<ORDER>& pf) {
-  constexpr int GT = MomX<ORDER>::GT, WIN = MomX<ORDER>::WIN;
-#pragma unroll
-  for (int j = 0; j < MomPf<ORDER>::NPF; j++) {
-    const int i = lt + GT * j;
-    if (i < WIN) wb[i] = pf.v[j];
-  }
-}
 
 // Per y-plane of an order: the number of x powers it feeds (always a prefix 0 .. npow - 1 of the powers) and the
 // moment-tile row of each, so that one plane body per power count serves every plane
@@ -927,34 +950,34 @@ __host__ __device__ constexpr int max_plane_powers(int order) {
 static_assert(max_plane_powers(1) == 3 && max_plane_powers(2) == 5, "the bodies' power counts");
 __constant__ PlaneRows c_plane_rows[2] = {build_plane_rows(1), build_plane_rows(2)};
 
-// one plane's x moments of powers 0 .. NP - 1 for a thread's RX pixels, from the segment in `wb`, into the tile rows mi
-template <int ORDER, int NP>
-__device__ __forceinline__ void mom_x_plane_np(const double* wb, double* mom, const int* mi, int lt, const MomTaps& tp) {
-  constexpr int R = MOM_R, RX = MomX<ORDER>::RX, SEG = MomX<ORDER>::SEG, NV = RX + 2 * R;
-  double v[NV];
-#pragma unroll
-  for (int i = 0; i < NV; i++) v[i] = wb[lt * RX + i];
-  double acc[RX][NP];
-#pragma unroll
-  for (int i = 0; i < RX; i++)
-#pragma unroll
-    for (int p = 0; p < NP; p++) acc[i][p] = p == 0 ? tp.k[0][0] * v[i + R] : 0.0;
-#pragma unroll
-  for (int t = 1; t <= R; t++)
-#pragma unroll
-    for (int i = 0; i < RX; i++) {
-      const double sp = v[i + R + t] + v[i + R - t], dm = v[i + R + t] - v[i + R - t];
-#pragma unroll
-      for (int p = 0; p < NP; p++) acc[i][p] = fma(tp.k[p][t], (p & 1) ? dm : sp, acc[i][p]);
+// the warps' y-planes: the most costly plane (2 + powers operations per tap pair) first, each to the least loaded warp
+template <int G>
+struct PlaneShare {
+  int n[G] = {};
+  int q[G][32] = {};
+};
+template <int G>
+__host__ __device__ constexpr PlaneShare<G> build_share(int order) {
+  PlaneShare<G> s{};
+  const PlaneRows r = build_plane_rows(order);
+  const int ny = build_table(order).ny;
+  int load[G] = {};
+  for (int np = 5; np >= 1; np--)
+    for (int q = 0; q < ny; q++) {
+      if (r.npow[q] != np) continue;
+      int g = 0;
+      for (int k = 1; k < G; k++)
+        if (load[k] < load[g]) g = k;
+      s.q[g][s.n[g]++] = q;
+      load[g] += np == 1 ? 2 : 2 + np;
     }
-#pragma unroll
-  for (int p = 0; p < NP; p++)
-#pragma unroll
-    for (int i = 0; i < RX; i++) mom[mi[p] * SEG + lt * RX + i] = acc[i][p];
+  return s;
 }
+__constant__ PlaneShare<MomX<1>::G> c_share1 = build_share<MomX<1>::G>(1);
+__constant__ PlaneShare<MomX<2>::G> c_share2 = build_share<MomX<2>::G>(2);
 
 template <int ORDER>
-__global__ void __launch_bounds__(MomX<ORDER>::NT, ORDER == 1 ? 4 : 2) k_moments_x_solve_rb(const double* __restrict__ yplanes,
+__global__ void __launch_bounds__(MomX<ORDER>::NT, MomX<ORDER>::MINB) k_moments_x_solve_rb(const double* __restrict__ yplanes,
                                                                const double* __restrict__ uxin,
                                                                const double* __restrict__ uyin, int W, int H,
                                                                MomTaps tp, double* __restrict__ oux,
@@ -962,42 +985,59 @@ __global__ void __launch_bounds__(MomX<ORDER>::NT, ORDER == 1 ? 4 : 2) k_moments
                                                                double* __restrict__ resid, double* __restrict__ slope) {
   constexpr MomTable T = build_table(ORDER);
   constexpr int n = ORDER == 1 ? 6 : 12;
-  constexpr int GT = MomX<ORDER>::GT, NT = MomX<ORDER>::NT, SEG = MomX<ORDER>::SEG, WIN = MomX<ORDER>::WIN;
+  constexpr int RX = MomX<ORDER>::RX, G = MomX<ORDER>::G, NT = MomX<ORDER>::NT, SEG = MomX<ORDER>::SEG;
+  constexpr int WIN = MomX<ORDER>::WIN, NI = WIN / 32;
   extern __shared__ double smd[];
-  double* mom = smd + 4 * WIN;
-  const int tid = threadIdx.x, g = tid / GT, lt = tid - g * GT, y = blockIdx.y, x0 = blockIdx.x * SEG;
+  double* mom = smd + 2 * G * WIN;
+  const int tid = threadIdx.x, g = tid >> 5, lane = tid & 31, y = blockIdx.y, x0 = blockIdx.x * SEG;
   const size_t N = (size_t)W * H;
-  MomPf<ORDER> pf;
-  if (g < T.ny) {  // group g's first plane into its buffer 0
-    mom_x_fetch<ORDER>(yplanes + (size_t)g * N + (size_t)y * W, x0, W, lt, pf);
-    mom_x_stage<ORDER>(smd + 2 * WIN * g, lt, pf);
-  }
-  __syncthreads();
-  // the plane pairs (K, K + 1): group g takes plane K + g from its buffer (K / 2) & 1, one body per power count
+  const auto& SH = [] () -> const auto& { if constexpr (ORDER == 1) return c_share1; else return c_share2; }();
   const PlaneRows& PR = c_plane_rows[ORDER - 1];
-  double* gb = smd + 2 * WIN * g;  // the group's two buffers
-#pragma unroll 1
-  for (int K = 0; K < T.ny; K += 2) {
-    const int Q = K + g;
-    const double* wb = gb + ((K / 2) & 1) * WIN;
-    double* wnext = gb + (((K / 2) + 1) & 1) * WIN;
-    if (Q + 2 < T.ny) mom_x_fetch<ORDER>(yplanes + (size_t)(Q + 2) * N + (size_t)y * W, x0, W, lt, pf);
-    if (Q < T.ny) {
-      int mi[5];
+  double* gb = smd + 2 * WIN * g;  // the warp's two buffers
+  int off[NI];                     // the lane's samples of a row segment, edges replicated
 #pragma unroll
-      for (int p = 0; p < 5; p++) mi[p] = PR.mi[Q][p];
-      const int np = PR.npow[Q];  // order 1: at most 3 (powers 0 .. 2); order 2: at most 5
-      if (np == 1) mom_x_plane_np<ORDER, 1>(wb, mom, mi, lt, tp);
-      else if (np == 2) mom_x_plane_np<ORDER, 2>(wb, mom, mi, lt, tp);
-      else if (ORDER == 1 || np == 3) mom_x_plane_np<ORDER, 3>(wb, mom, mi, lt, tp);
-      else if constexpr (ORDER > 1) {
-        if (np == 4) mom_x_plane_np<ORDER, 4>(wb, mom, mi, lt, tp);
-        else mom_x_plane_np<ORDER, 5>(wb, mom, mi, lt, tp);
-      }
+  for (int i = 0; i < NI; i++) off[i] = min(max(x0 - MOM_R + lane + 32 * i, 0), W - 1);
+  const int cnt = SH.n[g];
+  auto fetch = [&](int k) {
+    if (k < cnt) {
+      const double* row = yplanes + (size_t)SH.q[g][k] * N + (size_t)y * W;
+      double* dst = gb + (k & 1) * WIN + lane;
+#pragma unroll
+      for (int i = 0; i < NI; i++) __pipeline_memcpy_async(dst + 32 * i, row + off[i], sizeof(double));
     }
-    if (Q + 2 < T.ny) mom_x_stage<ORDER>(wnext, lt, pf);
-    __syncthreads();
+    __pipeline_commit();
+  };
+  fetch(0);
+#pragma unroll 1
+  for (int k = 0; k < cnt; k++) {
+    fetch(k + 1);
+    __pipeline_wait_prior(1);
+    __syncwarp();
+    const int q = SH.q[g][k];
+    const double* wb = gb + (k & 1) * WIN + lane * RX;
+    auto run = [&](auto npc) {
+      constexpr int NP = decltype(npc)::value;
+      double acc[RX][NP];
+      mom_slide<RX, NP>([&](int i) { return wb[i]; }, tp, acc);
+#pragma unroll
+      for (int p = 0; p < NP; p++) {
+        double* o = mom + PR.mi[q][p] * SEG + lane * RX;
+#pragma unroll
+        for (int j = 0; j < RX; j++) o[j] = acc[j][p];
+      }
+    };
+    const int np = PR.npow[q];  // order 1: at most 3 (powers 0 .. 2); order 2: at most 5
+    if (np == 1) run(std::integral_constant<int, 1>{});
+    else if (np == 2) run(std::integral_constant<int, 2>{});
+    else if (ORDER == 1 || np == 3) run(std::integral_constant<int, 3>{});
+    else if constexpr (ORDER > 1) {
+      if (np == 4) run(std::integral_constant<int, 4>{});
+      else run(std::integral_constant<int, 5>{});
+    }
+    __syncwarp();  // the buffer of plane k is free for plane k + 2
   }
+  __pipeline_wait_prior(0);
+  __syncthreads();
 #pragma unroll 1
   for (int s = tid; s < SEG; s += NT) {
     const int x = x0 + s;
@@ -1049,8 +1089,8 @@ template <int ORDER>
 static void launch_moments_rb(const double* sums, const double* ux, const double* uy, int W, int H, const MomTaps& tp,
                               double* yplanes, double* oux, double* ouy, double* energy, double* resid, double* slope,
                               cudaStream_t st) {
-  dim3 gy(div_up(W, 128), div_up(H, MOM_RY));
-  OFC_LAUNCH(k_moments_y_rb<ORDER>, gy, 128, 0, st, sums, W, H, tp, yplanes);
+  dim3 gy(div_up(W, 32), div_up(H, MY_W * MomY<ORDER>::RY), 7);
+  OFC_LAUNCH(k_moments_y_rb<ORDER>, gy, 32 * MY_W, 0, st, sums, W, H, tp, yplanes);
   const size_t sm = MomX<ORDER>::smem();
   raise_smem_limit((const void*)k_moments_x_solve_rb<ORDER>, sm);
   dim3 gx(div_up(W, MomX<ORDER>::SEG), H);

@@ -165,6 +165,24 @@ def test_local_solve(T, oracle, order):
         np.testing.assert_allclose(a, b, rtol=1e-7, atol=1e-9)
 
 
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("h,w", [(3, 5), (31, 32), (33, 96), (47, 97), (48, 159), (49, 161), (97, 193)])
+def test_local_solve_tile_edges(T, oracle, order, h, w):
+    """The window moments and the solve at the edges of their tiles: 32 columns x 48 (order 2: 32) rows in y, 160 (96)
+    pixels in x, images smaller than the window; the tolerance of test_local_solve."""
+    rng = np.random.default_rng(100 * h + w + order)
+    gx, gy = rng.normal(size=(2, 12, h, w))
+    wk = rng.uniform(0.1, 1.0, size=(12, h, w))
+    c = rng.normal(size=(12, h, w)) + 20.0
+    sums = [(wk * gx * gx).sum(0), (wk * gx * gy).sum(0), (wk * gy * gy).sum(0), (wk * gx * c).sum(0),
+            (wk * gy * c).sum(0), (wk * c * c).sum(0), wk.sum(0)]
+    ux, uy = rng.normal(size=(2, h, w))
+    got = T.local_solve(sums, ux, uy, Config(shape_order=order))
+    want = oracle.local_solve(sums, ux, uy, 4.0, order)
+    for a, b in zip(got, want):
+        np.testing.assert_allclose(a, b, rtol=1e-7, atol=1e-9)
+
+
 def test_median(T):
     rng = np.random.default_rng(5)
     for n in (1, 2, 3, 10, 1001, 4096, 100000):
