@@ -8,6 +8,7 @@ linked statically so the library needs only the driver on the machine that loads
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -47,7 +48,7 @@ def build(verbose=False, force=False):
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
     inc_dir = os.path.join(os.path.dirname(HERE), "include")
     headers += [os.path.join(inc_dir, f) for f in os.listdir(inc_dir) if f.endswith(".h")]
-    objs = []
+    objs, cmds = [], []
     for s in SOURCES:
         src = os.path.join(CSRC, s)
         obj = os.path.join(objdir, s.replace(".cu", ".o"))
@@ -55,7 +56,9 @@ def build(verbose=False, force=False):
         if force or _newer(obj, [src] + headers):
             inc = ["-I" + cutlass_include(), "-diag-suppress", "20012"] if s in CUTLASS_SOURCES else []
             cmd = [NVCC] + FLAGS + inc + (["-Xptxas", "-v"] if verbose else []) + ["-c", src, "-o", obj]
-            subprocess.run(cmd, check=True)
+            cmds.append(cmd)
+    with ThreadPoolExecutor(max(1, min(len(cmds), os.cpu_count() or 1))) as pool:
+        list(pool.map(lambda c: subprocess.run(c, check=True), cmds))
     if force or _newer(LIB, objs):
         subprocess.run([NVCC, "-shared", "-cudart", "static", "-gencode", "arch=compute_100a,code=sm_100a",
                         "-o", LIB] + objs, check=True)

@@ -351,23 +351,13 @@ struct Lane {
     auto it = plans.find(L);
     if (it != plans.end()) return it->second.first;
     FftPlan pl = fft_make_plan(L);
-    // twiddles of the stages' length, then (Bluestein) the chirp and the filter
-    std::vector<float2> tw = fft_twiddles(fft_work_len(pl));
-    const size_t ntw = tw.size();
-    if (pl.M) {
-      std::vector<float2> bt = fft_bluestein_tables(L, pl.M);
-      tw.insert(tw.end(), bt.begin(), bt.end());
-    }
+    std::vector<float2> tw = fft_tables(pl);
     std::unique_ptr<DevBuf> b(new DevBuf());
     size_t b32 = tw.size() * sizeof(float2);
     OFC_CUDA(cudaMalloc(&b->p, b32));
     b->bytes = b32;
     OFC_CUDA(cudaMemcpy(b->p, tw.data(), b32, cudaMemcpyHostToDevice));
-    pl.tw = (const float2*)b->p;
-    if (pl.M) {
-      pl.chirp = pl.tw + ntw;
-      pl.filt = pl.chirp + L;
-    }
+    fft_bind(pl, (const float2*)b->p);
     auto& slot = plans[L];
     slot.first = pl;
     slot.second = std::move(b);
@@ -3565,18 +3555,8 @@ int ofc_fft_tune(ofc_engine* e, const int32_t* lengths, size_t n, int lines, int
             ok = false;
           }
           if (ok) {
-            std::vector<float2> tw = fft_twiddles(fft_work_len(pl));
-            const size_t ntw = tw.size();
-            if (pl.M) {
-              std::vector<float2> bt2 = fft_bluestein_tables(L, pl.M);
-              tw.insert(tw.end(), bt2.begin(), bt2.end());
-            }
-            float2* dtw = Ln.upload("tune_tw", tw.data(), tw.size());
-            pl.tw = dtw;
-            if (pl.M) {
-              pl.chirp = pl.tw + ntw;
-              pl.filt = pl.chirp + L;
-            }
+            std::vector<float2> tw = fft_tables(pl);
+            fft_bind(pl, Ln.upload("tune_tw", tw.data(), tw.size()));
             float2* d = Ln.get<float2>("tune_lines", (size_t)lines * L);
             OFC_CUDA(cudaMemsetAsync(d, 0, (size_t)lines * L * sizeof(float2), Ln.stream));
             launch_fft_lines(d, lines, pl, false, Ln.stream);

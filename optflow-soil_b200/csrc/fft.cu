@@ -189,7 +189,8 @@ FftPlan fft_make_plan(int L, int variant) {
   FftPlan pl;
   pl.L = L;
   pl.M = work == L ? 0 : work;
-  std::vector<int> f = factor_order(work, variant);
+  // the plans fixed at compile time keep the default order
+  std::vector<int> f = factor_order(work, fft_fixed_length(work) || work == FFT_FIXED_M ? 0 : variant);
   if (f.empty() || (int)f.size() > FFT_MAXST)
     throw Error(OFC_ERR_WINDOW, "FFT length " + std::to_string(L) + " needs too many stages");
   int s = 1;
@@ -201,7 +202,41 @@ FftPlan fft_make_plan(int L, int variant) {
     pl.magic[i] = s == 1 ? 0u : (unsigned)((((unsigned long long)1 << 32) + s - 1) / s);
     s *= f[i];
   }
+  for (int i = 0, o = 0; i < pl.nst; i++) {
+    pl.so[i] = o;
+    o += (pl.p[i] - 1) * (work / (pl.p[i] * pl.s[i]));
+  }
   return pl;
+}
+
+std::vector<float2> fft_tables(const FftPlan& pl) {
+  const int SL = fft_work_len(pl);
+  const std::vector<float2> tw = fft_twiddles(SL);
+  std::vector<float2> out = tw;
+  for (int i = 0; i < pl.nst; i++) {
+    const int m = SL / (pl.p[i] * pl.s[i]);
+    for (int k = 1; k < pl.p[i]; k++)
+      for (int q = 0; q < m; q++) out.push_back(tw[(size_t)k * q * pl.s[i]]);
+  }
+  const size_t n = out.size() - SL;  // the inverse transform's conjugates
+  for (size_t i = 0; i < n; i++) out.push_back(make_float2(out[SL + i].x, -out[SL + i].y));
+  if (pl.M) {
+    const std::vector<float2> bt = fft_bluestein_tables(pl.L, pl.M);
+    out.insert(out.end(), bt.begin(), bt.end());
+  }
+  return out;
+}
+
+void fft_bind(FftPlan& pl, const float2* d) {
+  const int SL = fft_work_len(pl);
+  pl.tw = d;
+  pl.stw = d + SL;
+  const int last = pl.nst - 1;
+  pl.nstw = pl.so[last] + (pl.p[last] - 1) * (SL / (pl.p[last] * pl.s[last]));
+  if (pl.M) {
+    pl.chirp = pl.stw + 2 * pl.nstw;
+    pl.filt = pl.chirp + pl.L;
+  }
 }
 
 std::vector<float2> fft_twiddles(int L) {
@@ -211,6 +246,27 @@ std::vector<float2> fft_twiddles(int L) {
     t[i] = make_float2((float)std::cos(a), (float)std::sin(a));
   }
   return t;
+}
+
+// threads of a block of a runtime plan: the count up to RT_T for which the stages' rounds of butterflies (weighted by
+// the butterfly's length) leave the fewest threads idle
+static int rt_threads(const FftPlan& pl, int C) {
+  const int SL = fft_work_len(pl);
+  int best = RT_T;
+  double bc = 1e30;
+  for (int T = 96; T <= RT_T; T += 32) {
+    double c = 0;
+    for (int i = 0; i < pl.nst; i++) {
+      const int nb = SL / pl.p[i] * C, rounds = (nb + T - 1) / T;
+      c += (double)rounds * (pl.p[i] * pl.p[i] / 2 + 16 * pl.p[i]);
+    }
+    c *= T + 32;  // more threads per block, fewer blocks per SM
+    if (c < bc * 0.999) {
+      bc = c;
+      best = T;
+    }
+  }
+  return best;
 }
 
 int fft_threads(int L, int C) {
@@ -410,6 +466,18 @@ __device__ __forceinline__ void odd_butterfly(Load in, bool inv, Emit emit) {
 constexpr int FFT_PAD = 4;
 __host__ __device__ constexpr int fft_buf_len(int L, int C) { return L * C + ((L * C) >> FFT_PAD) + 1; }
 
+// Shared memory by 32-bit addresses: the stages are functions of their own, and through a generic pointer each of their
+// accesses would cost 64-bit address arithmetic and the generic path.
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ float2 lds2(unsigned a) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts2(unsigned a, float2 v) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+
 // The butterfly of radix P (P = 0: a direct DFT of runtime radix RP) on inputs in(j), j < P, with outputs
 // through emit(k, value) (which applies the inter-stage twiddle); tw_m(m) = w_P^m for the direct DFT.
 template <int P, class C2, class In, class Emit, class TwM>
@@ -474,83 +542,124 @@ __device__ __forceinline__ void butterfly(In in, Emit emit, TwM tw_m, int RP, bo
   }
 }
 
-// One Stockham stage of radix P from buffer A (layout shift ish) to buffer B (layout shift osh); C interleaved
-// lines of length L, C = 1 << lc. q, r of a butterfly come from multiplications by precomputed reciprocals
-// (magic = ceil(2^32 / s), exact for the sizes here). Radices 2, 4, 8 have hand-written butterflies, 3, 5, 7,
-// 11 and 13 the symmetric odd form, and any other radix (P = 0 here) a direct DFT with its inputs read from
-// shared memory. Each radix is its own non-inlined function, so that the registers of one radix's butterfly do
-// not add to another's. Butterfly b reads elements b + j istep (b = bi C + l with bi = q s + r).
-template <int P, class C2>
-__device__ __noinline__ void stage_loop(const C2* __restrict__ A, C2* __restrict__ B, int lc, int L, int Pr, int s,
-                                        unsigned magic, const C2* __restrict__ tw, bool inv, int ish, int osh) {
+// One Stockham stage of radix P from buffer A to buffer B; C interleaved lines of length L, C = 1 << LC. q of a butterfly
+// comes from a multiplication by a precomputed reciprocal (magic = ceil(2^32 / s), exact for the sizes here). Radices 2,
+// 4, 8 have hand-written butterflies, 3 ... 19 the symmetric odd form, and any other radix (P = 0 here) a direct DFT with
+// its inputs read from shared memory. Each radix is its own non-inlined function, so that the registers of one radix's
+// butterfly do not add to another's. Butterfly b reads elements b + j istep (b = bi C + l with bi = q s + r). ISH, OSH:
+// A, B in the padded layout (only a stage of an even radix with s C < 32 writes it: an odd radix's outputs fall on
+// distinct banks as they are). IN, OUT: what the first stage does to its inputs and the last to its outputs.
+enum FftIn { IN_PLAIN, IN_CHIRP, IN_MUL, IN_MULCHIRP };
+enum FftOut { OUT_PLAIN, OUT_FILT, OUT_CHIRP };
+// the operands of IN and OUT: Bluestein's chirp w (values i < L; a line's elements beyond L are 0) and filter f, the
+// conjugations of its inverse form, and the responses' factor (hx + omx omy) exb ey by of a column pair (row table yt of
+// (omy, ey by))
+struct StageEx {
+  int L;
+  bool conj;
+  const float2* w;
+  const float2* f;
+  const float2* yt;
+  float hx, omx, exb;
+};
+
+template <int IN>
+__device__ __forceinline__ float2 stage_in(unsigned a, int i, int lc, const StageEx& ex) {
+  if constexpr (IN == IN_PLAIN) return lds2(a);
+  const int e = i >> lc;
+  float2 v = make_float2(0.f, 0.f);
+  if (IN == IN_MUL || e < ex.L) {
+    v = lds2(a);
+    if constexpr (IN == IN_MUL || IN == IN_MULCHIRP) {  // the product rounded by itself (no contraction)
+      const float2 t = __ldg(ex.yt + e);
+      const float G = fmaf(ex.hx, t.x, ex.omx) * ex.exb * t.y;
+      v = make_float2(__fmul_rn(v.x, G), __fmul_rn(v.y, G));
+    }
+    if constexpr (IN == IN_CHIRP || IN == IN_MULCHIRP) {
+      if (ex.conj) v.y = -v.y;
+      v = cmul(v, __ldg(ex.w + e));
+    }
+  }
+  return v;
+}
+
+template <int P, int LC, int IN, int OUT, bool ISH, bool OSH>
+__device__ __noinline__ void stage_loop(unsigned A, unsigned B, int Pr, int s, int m,
+                                        unsigned magic, const float2* __restrict__ stw, const float2* __restrict__ tw,
+                                        bool inv, StageEx ex) {
   const int RP = P ? P : Pr;
-  const int C = 1 << lc;
-  const int m = L / (RP * s);
-  const int nb = (L / RP) << lc;
-  const int LP = L / RP;
-  const int istep = s * m * C, ostep = s * C;
+  constexpr int C = 1 << LC;
+  const int LP = s * m;  // L / RP
+  const int nb = LP << LC, istep = nb, ostep = s << LC;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    const int l = b & (C - 1), bi = b >> lc;
-    const int q = s == 1 ? bi : (int)__umulhi((unsigned)bi, magic), r = bi - q * s;
-    const int ob = (r + s * RP * q) * C + l;
+    const int l = b & (C - 1), bi = b >> LC;
+    const int q = s == 1 ? bi : (m == 1 ? 0 : (int)__umulhi((unsigned)bi, magic));
+    const int ob = ((bi + (RP - 1) * q * s) << LC) + l;
     auto in = [&](int j) {
       const int i = b + j * istep;
-      return A[i + (i >> ish)];
+      return stage_in<IN>(A + 8u * (unsigned)(ISH ? i + (i >> FFT_PAD) : i), i, LC, ex);
     };
-    auto emit = [&](int k, C2 val) {
-      if (k > 0 && q > 0) {
-        C2 w = __ldg(tw + (size_t)k * q * s);  // k q s < L
-        val = cmul(val, inv ? conjf2(w) : w);
+    auto emit = [&](int k, float2 val) {
+      if (OUT == OUT_PLAIN && k > 0 && q > 0) {
+        val = cmul(val, __ldg(stw + (k - 1) * m + q));
       }
       const int o = ob + k * ostep;
-      B[o + (o >> osh)] = val;
+      if constexpr (OUT == OUT_FILT) val = cmul(val, __ldg(ex.f + (o >> LC)));
+      if constexpr (OUT == OUT_CHIRP) {
+        if ((o >> LC) >= ex.L) return;
+        val = cmul(val, __ldg(ex.w + (o >> LC)));
+        if (ex.conj) val.y = -val.y;
+      }
+      sts2(B + 8u * (unsigned)(OSH ? o + (o >> FFT_PAD) : o), val);
     };
     auto tw_m = [&](int mm) {  // w_P^mm
-      C2 w = __ldg(tw + (size_t)mm * LP);
+      const float2 w = __ldg(tw + (size_t)mm * LP);
       return inv ? conjf2(w) : w;
     };
-    butterfly<P, C2>(in, emit, tw_m, RP, inv);
+    butterfly<P, float2>(in, emit, tw_m, RP, inv);
   }
 }
 
 // The same stage with every size known at compile time (radix P, stride S, length L, lines C, layout shifts):
-// the quotients, strides and padded offsets fold into constants.
-template <int P, int S, int L, int C, int ISH, int OSH, class C2>
-__device__ __noinline__ void stage_fixed(const C2* __restrict__ A, C2* __restrict__ B, const C2* __restrict__ tw,
-                                         bool inv) {
+// the quotients, strides and padded offsets fold into constants. IN, OUT: as in stage_loop. stw: the stage's twiddles of
+// the transform's direction.
+template <int P, int S, int L, int C, int ISH, int OSH, int IN, int OUT>
+__device__ __noinline__ void stage_fixed(unsigned A, unsigned B, const float2* __restrict__ stw, bool inv, StageEx ex) {
   constexpr int PB =
       (P == 2 || P == 3 || P == 4 || P == 5 || P == 7 || P == 8 || P == 11 || P == 13 || P == 17 || P == 19) ? P : 0;
-  constexpr int M = L / (P * S), NB = (L / P) * C, ISTEP = S * M * C, OSTEP = S * C, LP = L / P;
+  static_assert(PB != 0, "a plan of the radices with butterflies");
+  constexpr int M = L / (P * S), NB = (L / P) * C, ISTEP = S * M * C, OSTEP = S * C, LC = C == 2 ? 1 : 0;
+  static_assert(IN == IN_PLAIN || ISTEP % C == 0, "an element's column is the thread's");
   for (int b = threadIdx.x; b < NB; b += blockDim.x) {
     const int l = b % C, bi = b / C;
     const int q = bi / S, r = bi - q * S;
     const int ob = (r + S * P * q) * C + l;
     auto in = [&](int j) {
       const int i = b + j * ISTEP;
-      if constexpr (ISH < 31) return A[i + (i >> ISH)];
-      else return A[i];
+      if constexpr (ISH < 31) return stage_in<IN>(A + 8u * (unsigned)(i + (i >> ISH)), i, LC, ex);
+      else return stage_in<IN>(A + 8u * (unsigned)i, i, LC, ex);
     };
-    auto emit = [&](int k, C2 val) {
-      if (k > 0 && q > 0) {
-        C2 w = __ldg(tw + k * S * q);  // k q S < L
-        val = cmul(val, inv ? conjf2(w) : w);
-      }
+    auto emit = [&](int k, float2 val) {
+      if (OUT == OUT_PLAIN && M > 1 && k > 0 && q > 0) val = cmul(val, __ldg(stw + (k - 1) * M + q));
       const int o = ob + k * OSTEP;
-      if constexpr (OSH < 31) B[o + (o >> OSH)] = val;
-      else B[o] = val;
+      if constexpr (OUT == OUT_FILT) val = cmul(val, __ldg(ex.f + o / C));
+      if constexpr (OUT == OUT_CHIRP) {
+        if (o / C >= ex.L) return;
+        val = cmul(val, __ldg(ex.w + o / C));
+        if (ex.conj) val.y = -val.y;
+      }
+      if constexpr (OSH < 31) sts2(B + 8u * (unsigned)(o + (o >> OSH)), val);
+      else sts2(B + 8u * (unsigned)o, val);
     };
-    auto tw_m = [&](int mm) {  // w_P^mm
-      C2 w = __ldg(tw + mm * LP);
-      return inv ? conjf2(w) : w;
-    };
-    butterfly<PB, C2>(in, emit, tw_m, P, inv);
+    auto tw_m = [&](int) { return make_float2(0.f, 0.f); };  // the direct DFT's, not reached
+    butterfly<PB, float2>(in, emit, tw_m, P, inv);
   }
 }
 
 // compile-time plan: the factorisation of fft_make_plan (8s, 4s, 2s, then odd primes up to 31)
 struct CPlan {
-  int nst = 0;
-  int p[FFT_MAXST] = {}, s[FFT_MAXST] = {};
+  int nst = 0, nstw = 0;
+  int p[FFT_MAXST] = {}, s[FFT_MAXST] = {}, so[FFT_MAXST] = {};  // so, nstw: the stages' twiddles as in FftPlan
 };
 constexpr CPlan cplan(int L) {
   CPlan c{};
@@ -566,171 +675,147 @@ constexpr CPlan cplan(int L) {
     c.p[i] = f[i];
     c.s[i] = st;
     st *= f[i];
+    c.so[i] = c.nstw;
+    c.nstw += (f[i] - 1) * (L / st);
   }
   c.nst = n;
   return c;
 }
 
-template <int L, int C, int ST, class C2>
-__device__ __forceinline__ C2* fft_run_fixed(C2* a, C2* b, const C2* tw, bool inv) {
+// the fixed plan of length L from stage ST on: stage 0 reads `first` through IN, the last stage writes through OUT; the
+// stages write b, a, b, ... (ST = 0: first may be a); returns the buffer holding the result
+template <int L, int C, int ST, int IN, int OUT>
+__device__ __forceinline__ float2* fft_run_fixed(const float2* first, float2* a, float2* b, const FftPlan& pl, bool inv,
+                                                 const StageEx& ex) {
   constexpr CPlan P = cplan(L);
   if constexpr (ST == P.nst) {
     return a;
   } else {
     constexpr int OSH = (ST + 1 < P.nst && P.s[ST] * C < 32) ? FFT_PAD : 31;
     constexpr int ISH = ST == 0 ? 31 : (P.s[ST - 1] * C < 32 ? FFT_PAD : 31);
-    stage_fixed<P.p[ST], P.s[ST], L, C, ISH, OSH, C2>(a, b, tw, inv);
+    stage_fixed<P.p[ST], P.s[ST], L, C, ISH, OSH, ST == 0 ? IN : (int)IN_PLAIN, ST + 1 == P.nst ? OUT : (int)OUT_PLAIN>(
+        smem_addr(first), smem_addr(b), pl.stw + P.so[ST] + (inv ? P.nstw : 0), inv, ex);
     __syncthreads();
-    return fft_run_fixed<L, C, ST + 1, C2>(b, a, tw, inv);
+    return fft_run_fixed<L, C, ST + 1, IN, OUT>(b, b, a, pl, inv, ex);
   }
 }
 
-// The first stage of a fixed-length inverse column transform of a column pair with the responses' factor folded into
-// its loads: element i is raw[i] G, G = (hx + omx omy) ex ey bx by with (omy, ey by) the row table's entry of row
-// i / 2 and hx, omx, exb = ex bx the factors of the thread's column, which stays fixed (blockDim and the stage's input
-// stride are even). The products are rounded as the separate multiply pass rounded them (no contraction into the
-// butterfly's additions), so the transform sees the same values without that pass's shared-memory round trip and
-// barrier.
-template <int P, int S, int L, int C, int OSH, class C2>
-__device__ __noinline__ void stage_fixed_mul(const C2* __restrict__ raw, C2* __restrict__ B, const C2* __restrict__ tw,
-                                             bool inv, const float2* __restrict__ yt, float hx, float omx, float exb) {
-  static_assert(C == 2 && S == 1, "the first stage of a column pair");
-  constexpr int PB =
-      (P == 2 || P == 3 || P == 4 || P == 5 || P == 7 || P == 8 || P == 11 || P == 13 || P == 17 || P == 19) ? P : 0;
-  constexpr int M = L / (P * S), NB = (L / P) * C, ISTEP = S * M * C, OSTEP = S * C, LP = L / P;
-  static_assert(ISTEP % 2 == 0, "an element's column is the thread's");
-  for (int b = threadIdx.x; b < NB; b += blockDim.x) {
-    const int l = b % C, bi = b / C;
-    const int q = bi / S, r = bi - q * S;
-    const int ob = (r + S * P * q) * C + l;
-    auto in = [&](int j) {
-      const int i = b + j * ISTEP;
-      const float2 t = __ldg(yt + (i >> 1));
-      const C2 sv = raw[i];
-      const float G = fmaf(hx, t.x, omx) * exb * t.y;
-      return mkc<C2>(__fmul_rn(sv.x, G), __fmul_rn(sv.y, G));
+// stage st of the plan from A (padded: ish) to B; returns whether B is padded
+template <int LC, int IN, int OUT>
+__device__ __forceinline__ bool fft_stage(const float2* A, float2* B, const FftPlan& pl, int st, int SL, bool inv, bool ish,
+                                          const StageEx& ex) {
+  const int P = pl.p[st], s = pl.s[st], m = SL / (P * s);
+  const bool osh = P % 2 == 0 && st + 1 < pl.nst && (s << LC) < 32;
+  auto go = [&](auto pc) {
+    constexpr int PP = decltype(pc)::value;
+    constexpr bool EVEN = PP == 2 || PP == 4 || PP == 8;
+    auto call = [&](auto ic, auto oc) {
+      constexpr bool IS = decltype(ic)::value && IN == IN_PLAIN, OS = decltype(oc)::value && EVEN && OUT == OUT_PLAIN;
+      stage_loop<PP, LC, IN, OUT, IS, OS>(smem_addr(A), smem_addr(B), P, s, m, pl.magic[st], pl.stw + pl.so[st] + (inv ? pl.nstw : 0), pl.tw, inv, ex);
     };
-    auto emit = [&](int k, C2 val) {
-      if (k > 0 && q > 0) {
-        C2 w = __ldg(tw + k * S * q);  // k q S < L
-        val = cmul(val, inv ? conjf2(w) : w);
-      }
-      const int o = ob + k * OSTEP;
-      if constexpr (OSH < 31) B[o + (o >> OSH)] = val;
-      else B[o] = val;
-    };
-    auto tw_m = [&](int mm) {  // w_P^mm
-      C2 w = __ldg(tw + mm * LP);
-      return inv ? conjf2(w) : w;
-    };
-    butterfly<PB, C2>(in, emit, tw_m, P, inv);
-  }
-}
-
-// the fixed-length transform of a column pair whose first stage reads the staged pair `raw` through the factor
-// (stage_fixed_mul into a), then the remaining stages between a and b; returns the buffer holding the result
-template <int L, int C, class C2>
-__device__ __forceinline__ C2* fft_run_fixed_mul(const C2* raw, C2* a, C2* b, const C2* tw, bool inv,
-                                                 const float2* yt, float hx, float omx, float exb) {
-  constexpr CPlan P = cplan(L);
-  static_assert(P.nst >= 2, "at least two stages");
-  constexpr int OSH = (1 < P.nst && P.s[0] * C < 32) ? FFT_PAD : 31;
-  stage_fixed_mul<P.p[0], P.s[0], L, C, OSH, C2>(raw, a, tw, inv, yt, hx, omx, exb);
-  __syncthreads();
-  return fft_run_fixed<L, C, 1, C2>(a, b, tw, inv);
-}
-
-template <class C2>
-__device__ __forceinline__ void fft_stage(const C2* __restrict__ A, C2* __restrict__ B, int lc, int L, int P, int s,
-                                          unsigned magic, const C2* __restrict__ tw, bool inv, int ish, int osh) {
+    if (ish) {
+      if (EVEN && osh) call(std::true_type{}, std::true_type{});
+      else call(std::true_type{}, std::false_type{});
+    } else {
+      if (EVEN && osh) call(std::false_type{}, std::true_type{});
+      else call(std::false_type{}, std::false_type{});
+    }
+  };
+  using std::integral_constant;
   switch (P) {
-    case 2: stage_loop<2, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 3: stage_loop<3, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 4: stage_loop<4, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 5: stage_loop<5, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 7: stage_loop<7, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 8: stage_loop<8, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 11: stage_loop<11, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 13: stage_loop<13, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 17: stage_loop<17, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    case 19: stage_loop<19, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
-    default: stage_loop<0, C2>(A, B, lc, L, P, s, magic, tw, inv, ish, osh); break;
+    case 2: go(integral_constant<int, 2>{}); break;
+    case 3: go(integral_constant<int, 3>{}); break;
+    case 4: go(integral_constant<int, 4>{}); break;
+    case 5: go(integral_constant<int, 5>{}); break;
+    case 7: go(integral_constant<int, 7>{}); break;
+    case 8: go(integral_constant<int, 8>{}); break;
+    case 11: go(integral_constant<int, 11>{}); break;
+    case 13: go(integral_constant<int, 13>{}); break;
+    case 17: go(integral_constant<int, 17>{}); break;
+    case 19: go(integral_constant<int, 19>{}); break;
+    default: go(integral_constant<int, 0>{}); break;
   }
   __syncthreads();
+  return osh;
+}
+
+// the plan's stages on their length SL (L, or Bluestein's M): the first reads `first` through IN, the last writes dst
+// through OUT, those between alternate between b and a (all unpadded at the ends). dst may be `first` or a with an odd
+// number of stages, b with an even one; a null dst takes that one, which is returned.
+template <int LC, int IN, int OUT>
+__device__ __forceinline__ float2* fft_stages(const float2* first, float2* a, float2* b, float2* dst, const FftPlan& pl,
+                                              int SL, bool inv, const StageEx& ex) {
+  if (!dst) dst = pl.nst & 1 ? (pl.nst == 1 ? b : a) : a;
+  if (pl.nst == 1) {
+    fft_stage<LC, IN, OUT_PLAIN>(first, dst, pl, 0, SL, inv, false, ex);
+    return dst;
+  }
+  bool ish = fft_stage<LC, IN, OUT_PLAIN>(first, b, pl, 0, SL, inv, false, ex);
+  float2 *x = b, *y = a;
+  for (int st = 1; st + 1 < pl.nst; st++) {
+    ish = fft_stage<LC, IN_PLAIN, OUT_PLAIN>(x, y, pl, st, SL, inv, ish, ex);
+    float2* t = x;
+    x = y;
+    y = t;
+  }
+  if (dst == x) dst = y;
+  fft_stage<LC, IN_PLAIN, OUT>(x, dst, pl, pl.nst - 1, SL, inv, ish, ex);
+  return dst;
+}
+
+// Bluestein (the plan's M > 0): X_k = w_k sum_n (x_n w_n) conj(w_{k - n}), w_n = exp(-i pi n^2 / L), the convolution
+// cyclic over M >= 2L - 1 by two length-M transforms; the inverse transform as conj(forward(conj(x))). The products by
+// the chirp and the filter are made as the transforms' first stages load and their last stages store. `first` holds the
+// line's L values (x C); a and b fft_buf_len(M, C) values each (first may be a); the result goes to dst (its L values;
+// may be `first`), or for a null dst to a or b.
+template <int LC, int IN>
+__device__ __forceinline__ float2* fft_bluestein(const float2* first, float2* a, float2* b, float2* dst, const FftPlan& pl,
+                                                 bool inv, StageEx ex) {
+  ex.L = pl.L;
+  ex.conj = inv;
+  ex.w = pl.chirp;
+  ex.f = pl.filt;
+  float2* r = fft_stages<LC, IN == IN_MUL ? IN_MULCHIRP : IN_CHIRP, OUT_FILT>(first, a, b, nullptr, pl, pl.M, false, ex);
+  return fft_stages<LC, IN_PLAIN, OUT_CHIRP>(r, r, r == a ? b : a, dst, pl, pl.M, true, ex);
+}
+
+// a runtime plan's transform of the line(s) in `first` (L values x C, not kept) with two scratch buffers of
+// fft_buf_len(work length, C); the result goes to dst, which is neither scratch buffer
+template <int FIXL, int LC>
+__device__ __forceinline__ void fft_run_to(const float2* first, float2* a, float2* b, float2* dst, const FftPlan& pl, bool inv) {
+  if constexpr (FIXL == -1) fft_bluestein<LC, IN_PLAIN>(first, a, b, dst, pl, inv, StageEx{});
+  else fft_stages<LC, IN_PLAIN, OUT_PLAIN>(first, a, b, dst, pl, pl.L, inv, StageEx{});
+}
+
+// Bluestein with the inner length FM fixed at compile time (L still read at run time); the result in a or b
+template <int FM, int C, int IN>
+__device__ __forceinline__ float2* fft_bluestein_fixed(const float2* first, float2* a, float2* b, const FftPlan& pl, bool inv,
+                                                       StageEx ex) {
+  ex.L = pl.L;
+  ex.conj = inv;
+  ex.w = pl.chirp;
+  ex.f = pl.filt;
+  float2* r = fft_run_fixed<FM, C, 0, IN == IN_MUL ? (int)IN_MULCHIRP : (int)IN_CHIRP, OUT_FILT>(first, a, b, pl, false, ex);
+  return fft_run_fixed<FM, C, 0, IN_PLAIN, OUT_CHIRP>(r, r, r == a ? b : a, pl, true, ex);
 }
 
 // runs the plan on buf (tmp: scratch of the same capacity, fft_buf_len(fft_work_len(pl), C)); buf holds the input
 // unpadded and the returned buffer the result unpadded. FIXL > 0: the length is FIXL and the plan is fixed at
 // compile time; FIXL = 0: a runtime plan transformed directly; FIXL = -1: a runtime Bluestein plan (kernels are
 // instantiated per FIXL, so that each carries only its own path's code and registers).
-// the plan's stages on their length SL (L, or Bluestein's M): a holds the input unpadded, the returned buffer the
-// result unpadded
-template <int C, class C2>
-__device__ C2* fft_stages(C2* a, C2* b, const FftPlan& pl, int SL, bool inv) {
-  constexpr int lc = C == 4 ? 2 : (C == 2 ? 1 : 0);
-  const C2* tw = (const C2*)pl.tw;
-  int ish = 31;
-  for (int st = 0; st < pl.nst; st++) {
-    const int osh = (st + 1 < pl.nst && pl.s[st] * C < 32) ? FFT_PAD : 31;
-    fft_stage<C2>(a, b, lc, SL, pl.p[st], pl.s[st], pl.magic[st], tw, inv, ish, osh);
-    ish = osh;
-    C2* t = a;
-    a = b;
-    b = t;
-  }
-  return a;
-}
-
-// Bluestein (the plan's M > 0): X_k = w_k sum_n (x_n w_n) conj(w_{k - n}), w_n = exp(-i pi n^2 / L), the convolution
-// cyclic over M >= 2L - 1 by two length-M transforms; the inverse transform as conj(forward(conj(x))). buf and tmp
-// hold fft_buf_len(M, C) values each. FM > 0: the inner length is FM, its two transforms on the plan fixed at compile
-// time (L still read at run time).
-template <int C, class C2, int FM = 0>
-__device__ __forceinline__ C2* fft_bluestein(C2* buf, C2* tmp, const FftPlan& pl, bool inv) {
-  constexpr int lc = C == 4 ? 2 : (C == 2 ? 1 : 0);
-  const int L = pl.L, M = FM > 0 ? FM : pl.M;
-  auto inner = [&](C2* a, C2* b, bool iv) {
-    if constexpr (FM > 0) return fft_run_fixed<FM, C, 0, C2>(a, b, (const C2*)pl.tw, iv);
-    else return fft_stages<C, C2>(a, b, pl, M, iv);
-  };
-  const float2* w = pl.chirp;
-  const float2* f = pl.filt;
-  for (int idx = threadIdx.x; idx < M * C; idx += blockDim.x) {
-    const int i = idx >> lc;
-    float2 v = make_float2(0.f, 0.f);
-    if (i < L) {
-      v = buf[idx];
-      if (inv) v.y = -v.y;
-      v = cmul(v, __ldg(w + i));
-    }
-    buf[idx] = v;
-  }
-  __syncthreads();
-  C2* r = inner(buf, tmp, false);
-  for (int idx = threadIdx.x; idx < M * C; idx += blockDim.x) r[idx] = cmul(r[idx], __ldg(f + (idx >> lc)));
-  __syncthreads();
-  C2* q = inner(r, r == buf ? tmp : buf, true);
-  for (int idx = threadIdx.x; idx < L * C; idx += blockDim.x) {
-    float2 v = cmul(q[idx], __ldg(w + (idx >> lc)));
-    if (inv) v.y = -v.y;
-    q[idx] = v;
-  }
-  __syncthreads();
-  return q;
-}
-
 template <int FIXL, int C, class C2>
 __device__ C2* fft_run(C2* buf, C2* tmp, const FftPlan& pl, bool inv) {
-  static_assert(C == 1 || C == 2 || C == 4, "C: a power of two up to 4");
+  static_assert(C == 1 || C == 2, "C: one line or a pair");
   static_assert(std::is_same<C2, float2>::value, "float32 transforms");
+  constexpr int LC = C == 2 ? 1 : 0;
   if constexpr (FIXL > 0) {
-    return fft_run_fixed<FIXL, C, 0, C2>(buf, tmp, (const C2*)pl.tw, inv);
+    return fft_run_fixed<FIXL, C, 0, IN_PLAIN, OUT_PLAIN>(buf, buf, tmp, pl, inv, StageEx{});
   } else if constexpr (FIXL == -1) {  // the kernels' instantiation for Bluestein plans (pl.M > 0)
-    return fft_bluestein<C, C2>(buf, tmp, pl, inv);
+    return fft_bluestein<LC, IN_PLAIN>(buf, buf, tmp, nullptr, pl, inv, StageEx{});
   } else if constexpr (FIXL < -1) {  // Bluestein with the inner length -FIXL fixed at compile time
-    return fft_bluestein<C, C2, -FIXL>(buf, tmp, pl, inv);
+    return fft_bluestein_fixed<-FIXL, C, IN_PLAIN>(buf, buf, tmp, pl, inv, StageEx{});
   } else {
-    return fft_stages<C, C2>(buf, tmp, pl, pl.L, inv);
+    return fft_stages<LC, IN_PLAIN, OUT_PLAIN>(buf, buf, tmp, nullptr, pl, pl.L, inv, StageEx{});
   }
 }
 
@@ -841,11 +926,14 @@ __device__ __forceinline__ int reflect_near(int i, int n) {
 // 2112 = 8 8 3 11; the plan fixed at compile time), and FIXL = -FFT_FIXED_M (Bluestein with that inner length fixed);
 // the launchers pick by the plan.
 
+// blocks per SM of the runtime plans' kernels (80 registers; two blocks at 128 registers took 0.472 ms, four at 64 0.60 ms
+// in the row pass below)
+constexpr int RT_MINB = 3;
 // buffer stride of the kernels that stage several lines: fft_buf_len rounded up to an even count (16-byte aligned)
 __host__ __device__ constexpr int fft_buf_stride(int L, int C) { return (fft_buf_len(L, C) + 1) & ~1; }
 
 template <int FIXL>
-__global__ void __launch_bounds__(FFT_TMAX, 2) k_fft_rows_fwd_real(const float* __restrict__ img, int W, int H,
+__global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? FFT_TMAX : RT_T, FIXL > 0 || FIXL < -1 ? 2 : RT_MINB) k_fft_rows_fwd_real(const float* __restrict__ img, int W, int H,
                                                                   FftPlan plw, int ph, float2* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* sm = (float2*)smraw;
@@ -868,7 +956,7 @@ __global__ void __launch_bounds__(FFT_TMAX, 2) k_fft_rows_fwd_real(const float* 
 constexpr int COLS_TMAX = 320;  // threads per block of the split column pass
 
 template <int C, int FIXL>
-__global__ void __launch_bounds__(COLS_TMAX, 3) k_fft_cols_fwd(const float2* Tin, FftPlan plh, int pw, float2* S) {
+__global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? COLS_TMAX : RT_T, 3) k_fft_cols_fwd(const float2* Tin, FftPlan plh, int pw, float2* S) {
   constexpr int LC = C == 4 ? 2 : (C == 2 ? 1 : 0);
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* A = (float2*)smraw;
@@ -908,39 +996,13 @@ __global__ void __launch_bounds__(COLS_TMAX, 3) k_fft_cols_fwd(const float2* Tin
 // A thread's column is fixed (blockDim is even), so the x factors are read once.
 constexpr int RESP_G = 4;
 
-// A[i] = raw[i] f(i, t_i) for the n values of a column pair, t_i the row table entry of element i (row i / 2). With
-// the length fixed (FIXL, blockDim = NT) the table loads of UN elements are issued together before their
-// multiplies, so that their latencies overlap.
-template <int FIXL, int NT, int UN, class T, class Fn>
-__device__ __forceinline__ void cols_multiply(int n, const T* __restrict__ tab, Fn f) {
-  if constexpr (FIXL > 0) {
-    constexpr int NI = (2 * FIXL + NT - 1) / NT;
-#pragma unroll
-    for (int m0 = 0; m0 < NI; m0 += UN) {
-      T tv[UN];
-#pragma unroll
-      for (int u = 0; u < UN; u++) {
-        const int i = threadIdx.x + NT * (m0 + u);
-        if (m0 + u < NI && i < 2 * FIXL) tv[u] = __ldg(tab + (i >> 1));
-      }
-#pragma unroll
-      for (int u = 0; u < UN; u++) {
-        const int i = threadIdx.x + NT * (m0 + u);
-        if (m0 + u < NI && i < 2 * FIXL) f(i, tv[u]);
-      }
-    }
-  } else {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) f(i, __ldg(tab + (i >> 1)));
-  }
-}
-
 // threads of the fixed-length column-pair kernel: the responses COLS_TMAX; the reference pack, whose float64 factors
 // take more time per element, one per radix-8 butterfly of the two columns (2 x 2112 / 8)
 constexpr int PAIR_T_REF = 544;
 template <bool REFPACK>
-constexpr int pair_threads(int fixl) { return fixl > 0 && REFPACK ? PAIR_T_REF : COLS_TMAX; }
+constexpr int pair_threads(int fixl) { return fixl > 0 && REFPACK ? PAIR_T_REF : (fixl == 0 || fixl == -1 ? RT_T : COLS_TMAX); }
 template <bool REFPACK, int FIXL>
-__global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), 2) k_fft_cols_pair(const float2* __restrict__ S, FftPlan plh, int pw,
+__global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), FIXL == 0 || FIXL == -1 ? RT_MINB : 2) k_fft_cols_pair(const float2* __restrict__ S, FftPlan plh, int pw,
                                                                 GaborTables g, int k0, int k1, float2* __restrict__ U) {
   constexpr int C = 2;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -992,19 +1054,16 @@ __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), 2) k_fft_cols_pai
     for (int k = blockIdx.y * RESP_G; k < kend; k++) {
       // G = (hx + omx omy) ex ey (bx by): the x factors of the thread's column, (omy, ey by) from the row table
       const float exb = __ldg(g.exf + (size_t)k * pw + x) * bx;
+      StageEx ex{};
+      ex.yt = g.yt2 + (size_t)k * ph;
+      ex.hx = hx;
+      ex.omx = omx;
+      ex.exb = exb;
       float2* r;
-      if constexpr (FIXL > 0) {
-        r = fft_run_fixed_mul<FIXL, C, float2>(raw, A, B, (const float2*)plh.tw, true, g.yt2 + (size_t)k * ph, hx,
-                                               omx, exb);
-      } else {
-        cols_multiply<FIXL, COLS_TMAX, 14>(n, g.yt2 + (size_t)k * ph, [&](int i, float2 t) {
-          const float2 sv = raw[i];
-          const float G = fmaf(hx, t.x, omx) * exb * t.y;
-          A[i] = make_float2(sv.x * G, sv.y * G);
-        });
-        __syncthreads();
-        r = fft_run<FIXL, C>(A, B, plh, true);
-      }
+      if constexpr (FIXL > 0) r = fft_run_fixed<FIXL, C, 0, IN_MUL, OUT_PLAIN>(raw, A, B, plh, true, ex);
+      else if constexpr (FIXL < -1) r = fft_bluestein_fixed<-FIXL, C, IN_MUL>(raw, A, B, plh, true, ex);
+      else if constexpr (FIXL == 0) r = fft_stages<1, IN_MUL, OUT_PLAIN>(raw, A, B, nullptr, plh, ph, true, ex);
+      else r = fft_bluestein<1, IN_MUL>(raw, A, B, nullptr, plh, true, ex);
       float2* idle = r == A ? B : A;
       bspline_edge_consts<C>(r, ph, (float4*)idle);  // the prefilter's edge terms along y, added by the store
       store_edges(r, (const float4*)idle, k);
@@ -1066,7 +1125,7 @@ __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), 2) k_fft_cols_pai
 // The same inverse column pass with one block per (C columns, plane) and no staged spectrum: the form for padded
 // heights whose column pair does not fit in shared memory beside the two transform buffers.
 template <int C, bool REFPACK, int FIXL>
-__global__ void __launch_bounds__(COLS_TMAX, 3) k_fft_cols_inv_filter(const float2* __restrict__ S, FftPlan plh, int pw,
+__global__ void __launch_bounds__(RT_T, 3) k_fft_cols_inv_filter(const float2* __restrict__ S, FftPlan plh, int pw,
                                                                       GaborTables g, int k0, float2* __restrict__ U) {
   constexpr int LC = C == 4 ? 2 : (C == 2 ? 1 : 0);
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1173,13 +1232,59 @@ __global__ void __launch_bounds__(FIXL > 0 ? 288 : FFT_TMAX, FIXL > 0 ? 3 : 2)
   __pipeline_wait_prior(0);
 }
 
+// The same pass for runtime plans (times of 1367 x 911, rows of 1431 values, Bluestein's M = 2873 = 13 13 17: 0.451 ms per
+// launch; 0.838 ms with the four buffers of M, uncoalesced twiddles and separate passes for the chirp and filter products):
+// a block takes one node row. The two raw lines keep buffers of L values and receive
+// their own results; only the two scratch buffers have the work length (Bluestein's M is about 2 L). More blocks fit per
+// SM than with four buffers of M and a prefetch of the next row, and blocks of at most RT_T threads (rt_threads) leave few
+// warps without a butterfly in the stages of large radices. Issue slots (55 %) and barriers bound it.
 template <int FIXL>
-__global__ void __launch_bounds__(FFT_TMAX, 2) k_fft_rows_inv_ref(const float2* __restrict__ U, FftPlan plw, int ph, int W,
-                                                               int H, int k0, float4* __restrict__ ref4,
+__global__ void __launch_bounds__(RT_T, RT_MINB) k_fft_rows_inv_resp_rt(const float2* __restrict__ U, FftPlan plw, int ph, int F,
+                                                                  float scale, float2* __restrict__ R) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int L = plw.L, nl = fft_buf_stride(L, 1), nb = fft_buf_stride(fft_work_len(plw), 1), row = blockIdx.x;
+  float2 *x0 = (float2*)smraw, *x1 = x0 + nl, *a = x1 + nl, *b = a + nb;
+  const int j = row / ph, y = row - j * ph;
+  for (int c = 0; c < 2; c++) {
+    const float2* src = U + ((size_t)min(2 * j + c, F - 1) * ph + y) * L;
+    float2* dst = c ? x1 : x0;
+    if (L % 2 == 0) {  // 16-byte chunks: the line starts on a 16-byte boundary
+      for (int i = threadIdx.x; i < L / 2; i += blockDim.x) __pipeline_memcpy_async(dst + 2 * i, src + 2 * i, 16);
+    } else {
+      for (int i = threadIdx.x; i < L; i += blockDim.x) __pipeline_memcpy_async(dst + i, src + i, 8);
+    }
+    __pipeline_commit();
+  }
+  float4 k[2];
+#pragma unroll 1
+  for (int c = 0; c < 2; c++) {
+    float2* x = c ? x1 : x0;
+    if (c == 0) __pipeline_wait_prior(1);  // line 1 may be in flight
+    else __pipeline_wait_prior(0);
+    __syncthreads();
+    fft_run_to<FIXL, 0>(x, a, b, x, plw, true);
+    bspline_edge_consts<1>(x, L, (float4*)a);  // the edge terms along x, added by the store
+    k[c] = *(const float4*)a;
+    __syncthreads();
+  }
+  float4* o = (float4*)R + (size_t)row * L;
+  for (int x = threadIdx.x; x < L; x += blockDim.x) {
+    const float2 p = bspline_edge_fix(x0[x], x, L, k[0]), q = bspline_edge_fix(x1[x], x, L, k[1]);
+    o[x] = make_float4(p.x * scale, p.y * scale, q.x * scale, q.y * scale);
+  }
+}
+
+template <int FIXL>
+__global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? FFT_TMAX : RT_T, FIXL > 0 || FIXL < -1 ? 2 : RT_MINB) k_fft_rows_inv_ref(const float2* __restrict__ U, FftPlan plw, int ph, int W,
+                                                               int H, int k0, int two, float4* __restrict__ ref4,
                                                                float* __restrict__ amp) {
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* sm = (float2*)smraw;
-  const int pw = FIXL > 0 ? FIXL : plw.L, nb = fft_buf_stride(FIXL > 0 ? FIXL : fft_work_len(plw), 1);
+  // runtime plans: rows of L values and two scratch buffers of the work length, the results written over the rows (one
+  // scratch buffer and a copy of each result where a direct plan's five buffers do not fit: two = 0)
+  constexpr bool RT = FIXL == 0 || FIXL == -1;
+  const int pw = FIXL > 0 ? FIXL : plw.L, wl = fft_buf_stride(FIXL > 0 ? FIXL : fft_work_len(plw), 1);
+  const int nb = RT ? fft_buf_stride(pw, 1) : wl;
   float2* t = sm + 3 * nb;
   const int y = blockIdx.x, kk = blockIdx.y, k = k0 + kk;  // y: row of the W x H crop
   const size_t plane = (size_t)ph * pw;
@@ -1199,12 +1304,19 @@ __global__ void __launch_bounds__(FFT_TMAX, 2) k_fft_rows_inv_ref(const float2* 
     else if (v == 1) __pipeline_wait_prior(1);
     else __pipeline_wait_prior(0);
     __syncthreads();
-    float2* res = fft_run<FIXL, 1>(sm + v * nb, t, plw, true);
-    if (res != sm + v * nb) {
-      for (int x = threadIdx.x; x < pw; x += blockDim.x) sm[v * nb + x] = res[x];
-      __syncthreads();
+    if (RT && (FIXL == -1 || two)) {
+      if constexpr (RT) fft_run_to<FIXL, 0>(sm + v * nb, t, t + wl, sm + v * nb, plw, true);
+      rr[v] = sm + v * nb;
+      continue;
     }
-    rr[v] = sm + v * nb;
+    if constexpr (FIXL != -1) {
+      float2* res = fft_run<FIXL, 1>(sm + v * nb, t, plw, true);
+      if (res != sm + v * nb) {
+        for (int x = threadIdx.x; x < pw; x += blockDim.x) sm[v * nb + x] = res[x];
+        __syncthreads();
+      }
+      rr[v] = sm + v * nb;
+    }
   }
   const double sc = 1.0 / ((double)ph * (double)pw);
   for (int x = threadIdx.x; x < W; x += blockDim.x) {
@@ -1224,7 +1336,7 @@ __global__ void __launch_bounds__(FFT_TMAX, 2) k_fft_rows_inv_ref(const float2* 
 }
 
 template <int FIXL>
-__global__ void __launch_bounds__(FFT_TMAX, 2) k_fft_lines(float2* data, FftPlan pl, int inv) {
+__global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? FFT_TMAX : RT_T, 2) k_fft_lines(float2* data, FftPlan pl, int inv) {
   extern __shared__ float2 sm[];
   const int L = FIXL > 0 ? FIXL : pl.L;
   float2* row = data + (size_t)blockIdx.x * L;
@@ -1309,8 +1421,11 @@ bool fft_fits(int ph, int pw) {
   }
 }
 
+// whether a plan runs on the kernels' runtime instantiations (FIXL 0 or -1)
+static bool runtime_plan(const FftPlan& pl) { return pl.M ? pl.M != FFT_FIXED_M : !fft_fixed_length(pl.L); }
+
 void launch_fft_rows_fwd_real(const float* img, int W, int H, const FftPlan& plw, int ph, float2* out, cudaStream_t st) {
-  int T = fft_threads(fft_work_len(plw), 1);
+  int T = runtime_plan(plw) ? rt_threads(plw, 1) : fft_threads(fft_work_len(plw), 1);
   size_t sm = 2 * fbytes(fft_work_len(plw), 1);
   by_plan(plw, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
@@ -1322,7 +1437,7 @@ void launch_fft_rows_fwd_real(const float* img, int W, int H, const FftPlan& plw
 static void cols_fwd(float2* T, const FftPlan& plh, int pw, cudaStream_t st) {
   constexpr int C = 2;
   const int wh = fft_work_len(plh);
-  int nt = std::min(fft_threads(wh, C), COLS_TMAX);
+  int nt = runtime_plan(plh) ? rt_threads(plh, C) : std::min(fft_threads(wh, C), COLS_TMAX);
   size_t sm_f = 2 * (size_t)fft_buf_stride(wh, C) * sizeof(float2);
   // in place: a block reads its C columns whole before it writes their spectrum back
   by_plan(plh, [&](auto fl) {
@@ -1339,7 +1454,7 @@ static void cols_inverse(const float2* S, const FftPlan& plh, int pw, const Gabo
                          cudaStream_t st) {
   constexpr int C = 2;
   const int ph = plh.L, wh = fft_work_len(plh);
-  int nt = std::min(fft_threads(wh, C), COLS_TMAX);
+  int nt = runtime_plan(plh) ? rt_threads(plh, C) : std::min(fft_threads(wh, C), COLS_TMAX);
   const size_t sm_p = smem_cols_pair(ph, wh);
   if (sm_p <= SMEM_MAX) {
     if (fft_fixed_length(ph)) nt = pair_threads<REFPACK>(ph);  // the block size the fixed-length kernel assumes
@@ -1370,16 +1485,30 @@ void launch_fft_cols_filters(float2* T, const FftPlan& plh, int pw, const GaborT
 }
 
 void launch_fft_rows_inv_resp(const float2* U, const FftPlan& plw, int ph, int F, float2* R, cudaStream_t st) {
-  const int T = fft_threads(fft_work_len(plw), 1);
-  const size_t sm = smem_rows_resp(fft_work_len(plw));
   const float scale = (float)(36.0 / ((double)ph * (double)plw.L));
   const int nrows = ((F + 1) / 2) * ph;
+  if (runtime_plan(plw)) {
+    const int T = rt_threads(plw, 1);
+    const size_t sm = (2 * (size_t)fft_buf_stride(plw.L, 1) + 2 * (size_t)fft_buf_stride(fft_work_len(plw), 1)) * sizeof(float2);
+    auto launch = [&](auto fl) {
+      constexpr int FL = decltype(fl)::value;
+      set_smem((const void*)k_fft_rows_inv_resp_rt<FL>, sm);
+      OFC_LAUNCH(k_fft_rows_inv_resp_rt<FL>, nrows, T, sm, st, U, plw, ph, F, scale, R);
+    };
+    if (plw.M) launch(std::integral_constant<int, -1>{});
+    else launch(std::integral_constant<int, 0>{});
+    return;
+  }
+  const int T = fft_threads(fft_work_len(plw), 1);
+  const size_t sm = smem_rows_resp(fft_work_len(plw));
   by_plan(plw, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
-    const void* fn = (const void*)k_fft_rows_inv_resp<FL>;
-    set_smem(fn, sm);
-    OFC_LAUNCH(k_fft_rows_inv_resp<FL>, persistent_blocks(fn, T, sm, nrows), T, sm, st, U, plw, ph, F, nrows, scale,
-               R);
+    if constexpr (FL > 0 || FL < -1) {
+      const void* fn = (const void*)k_fft_rows_inv_resp<FL>;
+      set_smem(fn, sm);
+      OFC_LAUNCH(k_fft_rows_inv_resp<FL>, persistent_blocks(fn, T, sm, nrows), T, sm, st, U, plw, ph, F, nrows, scale,
+                 R);
+    }
   });
 }
 
@@ -1392,18 +1521,23 @@ void launch_fft_cols_ref_f32(const float2* S, const FftPlan& plh, int pw, const 
 
 void launch_fft_rows_inv_ref_f32(const float2* U, const FftPlan& plw, int ph, int k0, int k1, int W, int H,
                                  float4* ref4, float* amp, cudaStream_t st) {
-  int T = fft_threads(fft_work_len(plw), 1);
-  size_t sm = 4 * (size_t)fft_buf_stride(fft_work_len(plw), 1) * sizeof(float2);
+  const bool rt = runtime_plan(plw);
+  const size_t wl = fft_buf_stride(fft_work_len(plw), 1);
+  int T = rt ? rt_threads(plw, 1) : fft_threads(fft_work_len(plw), 1);
+  size_t sm = 4 * wl * sizeof(float2);
+  const size_t sm2 = (3 * (size_t)fft_buf_stride(plw.L, 1) + 2 * wl) * sizeof(float2);
+  const bool two = rt && sm2 <= SMEM_MAX;
+  if (two) sm = sm2;
   dim3 grid(H, k1 - k0);
   by_plan(plw, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
     set_smem((const void*)k_fft_rows_inv_ref<FL>, sm);
-    OFC_LAUNCH(k_fft_rows_inv_ref<FL>, grid, T, sm, st, U, plw, ph, W, H, k0, ref4, amp);
+    OFC_LAUNCH(k_fft_rows_inv_ref<FL>, grid, T, sm, st, U, plw, ph, W, H, k0, two ? 1 : 0, ref4, amp);
   });
 }
 
 void launch_fft_lines(float2* data, int lines, const FftPlan& pl, bool inverse, cudaStream_t st) {
-  int T = fft_threads(fft_work_len(pl), 1);
+  int T = runtime_plan(pl) ? rt_threads(pl, 1) : fft_threads(fft_work_len(pl), 1);
   size_t sm = 2 * fbytes(fft_work_len(pl), 1);
   by_plan(pl, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;

@@ -17,9 +17,13 @@ bool fft_fixed_length(int L);
 constexpr int FFT_FIXED_M = 1216;
 constexpr int FFT_E = 8;       // complex values per thread (sets the threads of a block)
 constexpr int FFT_TMAX = 512;  // threads per block at most
+constexpr int RT_T = 256;      // the same of the runtime plans' kernels
 
 // A 1-D plan of length L: mixed-radix Stockham stages (radix p[i], stride s[i] = product of the radices
-// before it) and the twiddle table W[t] = exp(-2 pi i t / L), t < L, rounded from float64.
+// before it) and the twiddle table W[t] = exp(-2 pi i t / L), t < L, rounded from float64. Stage i's twiddles lie together
+// as its butterflies read them, stw[so[i] + (k - 1) m + q] = W[k q s[i]] (m = L / (p[i] s[i]), k = 1 .. p[i] - 1, q < m):
+// neighbouring threads (consecutive q) read neighbouring values, where W itself is read at a stride of k s[i]; the nstw
+// values are followed by their conjugates (the inverse transform's).
 // A length with a prime factor above 31 is transformed by Bluestein's chirp z-transform (as the reference's Metal
 // FFT does, rust/crates/optflow-gpu/src/fft.rs:1-3): M > 0 is then the inner length (a length >= 2L - 1 of
 // the radices with butterflies, of fewest stages: fft_work_length), the stages and tw are those of length M, chirp[n] = exp(-i pi n^2 / L) for n < L, and filt is the
@@ -30,7 +34,10 @@ struct FftPlan {
   int p[FFT_MAXST] = {};
   int s[FFT_MAXST] = {};
   unsigned magic[FFT_MAXST] = {};
+  int so[FFT_MAXST] = {};
   const float2* tw = nullptr;
+  const float2* stw = nullptr;
+  int nstw = 0;
   int M = 0;
   const float2* chirp = nullptr;
   const float2* filt = nullptr;
@@ -45,8 +52,7 @@ bool fft_supported(int L);
 int fft_work_length(int L);
 // whether the column and row passes of a ph x pw padded window fit in shared memory
 bool fft_fits(int ph, int pw);
-// host: factor L (or Bluestein's M) and fill p/s; the caller sets tw (fft_twiddles(fft_work_length(L))) and, for
-// Bluestein, chirp and filt (fft_bluestein_tables: L chirp values, then M filter values)
+// host: factor L (or Bluestein's M) and fill p/s; the caller uploads fft_tables and binds them (fft_bind)
 FftPlan fft_make_plan(int L);
 // the plan with a given factor order (0 .. FFT_PLAN_VARIANTS - 1); fft_make_plan(L) takes the plan table's choice
 constexpr int FFT_PLAN_VARIANTS = 4;
@@ -57,6 +63,10 @@ void fft_set_plan_variant(int L, int variant);
 int fft_plan_variant(int L);
 std::vector<float2> fft_twiddles(int L);
 std::vector<float2> fft_bluestein_tables(int L, int M);
+// every table of a plan in one vector (twiddles, stage twiddles and, for Bluestein, the chirp and the filter), and the
+// binding of the plan to a device copy of it
+std::vector<float2> fft_tables(const FftPlan& pl);
+void fft_bind(FftPlan& pl, const float2* d);
 // threads of a block that transforms C interleaved lines of length L (multiple of C and of 32)
 int fft_threads(int L, int C);
 

@@ -24,6 +24,29 @@ def T():
 BLUESTEIN = [37, 164, 106, 604, 191, 1021, 1999]
 
 
+@pytest.mark.parametrize("L,bound", [(144, 2e-6), (441, 2e-6), (650, 2e-6), (975, 2e-6), (1539, 2e-6), (2023, 2e-6),
+                                      (2048, 2e-6), (253, 2e-6), (397, 1e-5), (433, 1e-5), (917, 1e-5), (1109, 1e-5),
+                                      (1431, 1e-5), (1822, 1e-5)])
+def test_fft_lines_runtime_plans(T, L, bound):
+    """Runtime plans by their stages' kinds: even radices first (padded stores), odd radices only, a radix above 19 (direct
+    DFT), Bluestein inner lengths of 2 and 3 stages of the large radices and of 4 stages; the bounds of
+    test_fft_lines_match_numpy."""
+    rng = np.random.default_rng(L)
+    a = (rng.standard_normal((3, L)) + 1j * rng.standard_normal((3, L))).astype(np.complex64)
+    for inv in (False, True):
+        got = T.fft_lines(a, inverse=inv)
+        ref = np.fft.ifft(a.astype(np.complex128), axis=1) * L if inv else np.fft.fft(a.astype(np.complex128), axis=1)
+        assert np.abs(got - ref).max() < bound * np.abs(ref).max(), (L, inv)
+
+
+@pytest.mark.parametrize("shape", [(133, 911), (40, 1367), (1367, 75), (185, 333), (40, 5936)])
+def test_passes_runtime_plans(T, oracle, shape):
+    """The row and column passes on runtime plans (direct, Bluestein, odd pitches; 6000 padded columns, where the
+    reference pack's rows have one scratch buffer): test_responses and test_reference_phase_fixed_length at these sizes."""
+    test_responses_fixed_length(T, oracle, shape)
+    test_reference_phase_fixed_length(T, shape)
+
+
 @pytest.mark.parametrize("L", [64, 128, 160, 192, 224, 320, 576, 832, 1024, 1088, 1152, 1600, 2112, 2*3*5*7*11, 3*17*19,
                                23*29, 31*8]
                          + BLUESTEIN)
