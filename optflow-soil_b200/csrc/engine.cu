@@ -622,7 +622,7 @@ FineOut refine_dev(Lane& L, const float* i1, int W, int H, const float* i2, int 
   int* cold2 = L.get<int>("col_d2", N);
   int* colrow = L.get<int>("col_row", N);
   PrewarpCounts* counts = L.get<PrewarpCounts>("pw_counts", 2);
-  OFC_CUDA(cudaMemsetAsync(hist, 0, 4096 * sizeof(unsigned long long), st));
+  launch_energy_stats_init(stats, hist, st);
   launch_fill_f64(resid, PI, N, st);
   launch_fill_f64(energy, 1.0, N, st);
   OFC_CUDA(cudaMemsetAsync(slope, 0, 4 * N * sizeof(double), st));
@@ -631,7 +631,7 @@ FineOut refine_dev(Lane& L, const float* i1, int W, int H, const float* i2, int 
   const int Kf = c.prewarp_freeze_at;
   double* ucur = u2;
   double* unext = u2b;
-  bool primed = false;  // the first median starts the select state itself; each reset primes the next one's
+  int half = 0;  // of the median state
   for (int it = 0; it < c.outer_iters; it++) {
     const double* blur_in = ucur;
     if (it > 0) {
@@ -669,10 +669,9 @@ FineOut refine_dev(Lane& L, const float* i1, int W, int H, const float* i2, int 
       launch_accumulate(ref4, R, F, ph, pw, ucur, ucur + N, s2, s2 + N, (const double2*)cs2, W, H, sums, st);
       launch_moments_solve(sums, ucur, ucur + N, W, H, c.shape_order, d_mt, rw, mtp, yplanes, unext, unext + N, energy,
                            resid, slope, st);
-      const bool last_inner = in == c.inner_iters - 1;
-      launch_energy_median(energy, N, stats, last_inner, hist, st, primed);
-      launch_reset(energy, ucur, ucur + N, (int)N, stats, unext, unext + N, resid, slope, st, true);
-      primed = true;
+      const bool last_inner = in == c.inner_iters - 1;  // the confidence reads the median
+      launch_median_reset(energy, N, stats, half, last_inner, hist, ucur, ucur + N, unext, unext + N, resid, slope, st);
+      half ^= 1;
       std::swap(ucur, unext);
     }
   }
@@ -3212,10 +3211,9 @@ int ofc_test_local_solve(ofc_engine* e, const double* sums, const double* ux, co
     double* yp = L.get<double>("yplanes", (size_t)moment_yplanes(c->shape_order) * N);
     EnergyStats* stats = L.get<EnergyStats>("stats", 1);
     unsigned long long* hist = L.get<unsigned long long>("hist", median_scratch(N));
-    OFC_CUDA(cudaMemsetAsync(hist, 0, 4096 * sizeof(unsigned long long), L.stream));
+    launch_energy_stats_init(stats, hist, L.stream);
     launch_moments_solve(ds, u2, u2 + N, W, H, c->shape_order, d_mt, rw, mtp, yp, o2, o2 + N, en, rs, sl, L.stream);
-    launch_energy_median(en, N, stats, false, hist, L.stream);
-    launch_reset(en, u2, u2 + N, (int)N, stats, o2, o2 + N, rs, sl, L.stream);
+    launch_median_reset(en, N, stats, 0, false, hist, u2, u2 + N, o2, o2 + N, rs, sl, L.stream);
     OFC_CUDA(cudaMemcpyAsync(oux, o2, N * 8, cudaMemcpyDeviceToHost, L.stream));
     OFC_CUDA(cudaMemcpyAsync(ouy, o2 + N, N * 8, cudaMemcpyDeviceToHost, L.stream));
     OFC_CUDA(cudaMemcpyAsync(energy, en, N * 8, cudaMemcpyDeviceToHost, L.stream));
@@ -3231,8 +3229,8 @@ int ofc_test_median(ofc_engine* e, const double* v, size_t n, double* median, ch
     double* d = L.upload("t_med", v, n);
     EnergyStats* stats = L.get<EnergyStats>("stats", 1);
     unsigned long long* hist = L.get<unsigned long long>("hist", median_scratch(n));
-    OFC_CUDA(cudaMemsetAsync(hist, 0, 4096 * sizeof(unsigned long long), L.stream));
-    launch_energy_median(d, n, stats, true, hist, L.stream);
+    launch_energy_stats_init(stats, hist, L.stream);
+    launch_median_reset(d, n, stats, 0, true, hist, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, L.stream);
     EnergyStats hs;
     OFC_CUDA(cudaMemcpyAsync(&hs, stats, sizeof(hs), cudaMemcpyDeviceToHost, L.stream));
     OFC_CUDA(cudaStreamSynchronize(L.stream));

@@ -1116,7 +1116,7 @@ void launch_moments_solve(const double* sums, const double* ux, const double* uy
   }
 }
 
-// ---------------------------------------------------------------- energy statistics and median
+// ---------------------------------------------------------------- the energies' range
 __device__ __forceinline__ unsigned long long okey(double v) {  // order-preserving key of a double
   unsigned long long u = (unsigned long long)__double_as_longlong(v);
   return (u >> 63) ? ~u : (u | 0x8000000000000000ULL);
@@ -1126,359 +1126,313 @@ __device__ __forceinline__ double okey_inv(unsigned long long k) {
   return __longlong_as_double((long long)u);
 }
 
-__device__ double atomic_min_d(double* a, double v) {
-  unsigned long long* p = (unsigned long long*)a;
-  unsigned long long old = *p, assumed;
-  while (v < __longlong_as_double(old)) {
-    assumed = old;
-    old = atomicCAS(p, assumed, __double_as_longlong(v));
-    if (old == assumed) break;
+
+// the range and NaN of a warp's energies (a thread's smallest and largest key, ~0 and 0 without one) into the state: an
+// atomic only where it improves what is there already
+__device__ __forceinline__ void energy_range(EnergyStats::Half* h, unsigned long long lo, unsigned long long hi, bool nan) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
+    lo = a < lo ? a : lo;
+    hi = b > hi ? b : hi;
   }
-  return __longlong_as_double(old);
-}
-__device__ double atomic_max_d(double* a, double v) {
-  unsigned long long* p = (unsigned long long*)a;
-  unsigned long long old = *p, assumed;
-  while (v > __longlong_as_double(old)) {
-    assumed = old;
-    old = atomicCAS(p, assumed, __double_as_longlong(v));
-    if (old == assumed) break;
+  nan = __any_sync(0xffffffffu, nan);
+  if ((threadIdx.x & 31) == 0) {
+    if (lo < __ldcg(&h->lo)) atomicMin(&h->lo, lo);
+    if (hi > __ldcg(&h->hi)) atomicMax(&h->hi, hi);
+    if (nan) atomicOr(&h->nan, 1u);
   }
-  return __longlong_as_double(old);
 }
 
-// ---- median of the energy (np.median, phaseflow.py:149-151): an exact radix select over order-preserving keys.
-// 1. k_stats_hist0: min / max / NaN (the reset rule, phaseflow.rs:846-854) and the histogram of the top 12 key bits
-//    in one scan; the last block decides whether the median is needed and picks the first digit.
-// 2. k_radix_hist pass 1: the next 12 bits among the elements of that bucket.
-// 3. k_radix_compact: the elements of the 24-bit bucket into a candidate list (room for all n), and the largest
-//    key below the bucket.
-// 4. k_radix_final (one block): the remaining 40 bits over the candidates, the largest key below the median's, and
-//    the median (the mean of the two middle values for even n).
-// Four or five launches per median whatever the data (k_stats_init first, unless the last k_reset primed the state);
-// a bucket of many equal energies (heavy ties) only makes the one-block final select longer.
-constexpr int RBITS = 12, RBINS = 1 << RBITS;
-constexpr int RH_T = 512;
+// ---------------------------------------------------------------- energy median and reset
+// The median of the energy (np.median, phaseflow.py:149-151) by an exact radix select over order-preserving keys, and the
+// reset that reads it, in one cooperative launch whose blocks meet at grid barriers:
+// 1. the range of the energies (barrier) and the reset rule (phaseflow.rs:846-854): when every energy is above
+//    1e-9 max + 1e-30 no pixel is reset, and unless the caller needs the median every block returns.
+// 2. a histogram of 4096 equal parts of the keys' range (barrier), from which every block picks the median's part;
+// 3. the elements of that part into a candidate list (room for all n) and the largest key below it (barrier);
+// 4. every block selects the median among the candidates (by counting where there are at most 1024, else by 12-bit
+//    digits) and resets its share of the pixels.
+// Small images are bound by the launches' latency, large ones by the scans. Five launches before (two histogram scans, the
+// compaction, the final select, the reset; 80 per refinement): 128^2 pairs 1.459 -> 1.214 ms, 2048^2 30.85 -> 30.36 ms.
+// Taking the range in the solve's epilogue saves the first scan and barrier but costs the solve registers (2048^2: 0.333
+// -> 0.357 ms per launch), more than it gives. A barrier gives up after MED_SPINS polls, the median is NaN then.
+// threads, parts, energies a thread keeps in registers (4: 1.257 ms per 128^2 pair, 16: 1.285, 8: 1.214), and the energies
+// per block below one block per SM
+constexpr int MED_T = 1024, MED_BINS = 4096, MED_E = 8, MED_PER = MED_T * MED_E;
+constexpr unsigned MED_SPINS = 1u << 22;
 
-// the select state a median starts from (median, need_median and skip_reset, which the median's readers use, are
-// left alone)
-__device__ __forceinline__ void stats_prime(EnergyStats* s, size_t n) {
-  s->lo = DBL_MAX;
-  s->hi = -DBL_MAX;
-  s->nan = 0;
-  s->prefix = 0;
-  s->rank = (long long)(n / 2);
-  s->less = 0;
-  s->ticket = 0;
-  s->lo_val = 0;
-  s->ncand = 0;
-  s->below_max = 0;
+__global__ void k_stats_init(EnergyStats* s) {
+  s->median = 0.0;
+  s->timeouts = 0;
+  for (int i = 0; i < 2; i++) s->half[i] = EnergyStats::Half{~0ull, 0ull, 0ull, 0u, 0u, 0u};
 }
 
-__global__ void k_stats_init(EnergyStats* s, size_t n) { stats_prime(s, n); }
-
-__device__ __forceinline__ void digit_of(int pass, int& shift, int& bits) {
-  int hi = 64 - RBITS * pass;
-  bits = hi >= RBITS ? RBITS : hi;
-  shift = hi - bits;
+// every block of the grid arrives for the `round`-th time; false where the wait gave up
+__device__ bool grid_meet(EnergyStats* s, EnergyStats::Half* h, unsigned round) {
+  if (gridDim.x == 1) {
+    __syncthreads();
+    return true;
+  }
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&h->bar, 1u);
+    const unsigned want = round * gridDim.x;
+    unsigned seen = 0, k = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&h->bar) : "memory");
+    } while (seen < want && ++k < MED_SPINS);
+    ok = seen >= want;
+    if (seen < want) atomicAdd(&s->timeouts, 1u);
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
 }
 
-// run by every thread of the last block of a histogram pass: scans the RBINS counts of hist, finds the bin that
-// holds rank, extends the prefix by it, and clears hist and the ticket for the next pass
-__device__ void radix_pick(unsigned long long* hist, EnergyStats* s, int shift, long long* wsum) {
-  constexpr int per = RBINS / RH_T;
+// the bin of 4096 counts (count(i)) that holds `rank`, and the number of elements in the bins before it; every thread of
+// the block gets both. total: at least rank + 1
+template <class Count>
+__device__ void block_pick(Count count, long long rank, int& bin, long long& before) {
+  constexpr int PER = MED_BINS / MED_T;
+  __shared__ long long wsum[MED_T / 32], sh_before;
+  __shared__ int sh_bin;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  long long c[per];
+  unsigned c[PER];
   long long loc = 0;
 #pragma unroll
-  for (int j = 0; j < per; j++) {
-    c[j] = (long long)__ldcg(hist + tid * per + j);
+  for (int j = 0; j < PER; j++) {
+    c[j] = count(tid * PER + j);
     loc += c[j];
   }
   long long inc = loc;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    long long v = __shfl_up_sync(0xffffffffu, inc, o);
+    const long long v = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += v;
   }
   if (lane == 31) wsum[wid] = inc;
   __syncthreads();
   if (wid == 0) {
-    long long w = lane < RH_T / 32 ? wsum[lane] : 0;
+    long long w = wsum[lane];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      long long v = __shfl_up_sync(0xffffffffu, w, o);
+      const long long v = __shfl_up_sync(0xffffffffu, w, o);
       if (lane >= o) w += v;
     }
-    if (lane < RH_T / 32) wsum[lane] = w;
+    wsum[lane] = w;
   }
   __syncthreads();
-  const long long excl = inc - loc + (wid ? wsum[wid - 1] : 0);
-  const long long rank = s->rank;
-  if (excl <= rank && rank < excl + loc) {  // exactly one thread
-    long long acc = excl;
-    int bin = tid * per;
+  long long acc = inc - loc + (wid ? wsum[wid - 1] : 0);
+  if (acc <= rank && rank < acc + loc) {  // exactly one thread
+    int j = 0;
 #pragma unroll
-    for (int j = 0; j < per; j++) {
-      if (acc + c[j] > rank) {
-        bin = tid * per + j;
-        break;
+    for (int i = 0; i < PER - 1; i++)
+      if (j == i && acc + c[i] <= rank) {
+        acc += c[i];
+        j = i + 1;
       }
-      acc += c[j];
-    }
-    s->prefix |= ((unsigned long long)bin) << shift;
-    s->rank = rank - acc;
-    s->less += acc;
+    sh_bin = tid * PER + j;
+    sh_before = acc;
   }
+  __syncthreads();
+  bin = sh_bin;
+  before = sh_before;
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(MED_T) k_median_reset(const double* __restrict__ e, size_t n, EnergyStats* s, int half,
+                                                      int force, unsigned* hist2, unsigned long long* cand,
+                                                      const double* __restrict__ uxin, const double* __restrict__ uyin,
+                                                      double* ux, double* uy, double* resid, double* slope) {
+  __shared__ unsigned h[MED_BINS];
+  __shared__ unsigned long long keys[MED_T];
+  __shared__ unsigned long long sh_key, sh_below;
+  __shared__ long long sh_less;
+  EnergyStats::Half& P = s->half[half];
+  unsigned* hist = hist2 + half * MED_BINS;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const size_t i0 = blockIdx.x * (size_t)MED_T + tid, step = (size_t)gridDim.x * MED_T;
+  unsigned round = 0;
+  // the other half's start state for the next solve and median (the launch that used it has ended)
+  for (size_t i = i0; i < MED_BINS; i += step) hist2[(half ^ 1) * MED_BINS + i] = 0;
+  if (i0 == 0) s->half[half ^ 1] = EnergyStats::Half{~0ull, 0ull, 0ull, 0u, 0u, 0u};
+  // a thread's first MED_E energies stay in registers (all of them up to MED_T MED_E per block), later ones are read again
+  double v[MED_E];
 #pragma unroll
-  for (int j = 0; j < per; j++) hist[tid * per + j] = 0;
-  if (tid == 0) s->ticket = 0;
-}
-
-// adds the block histogram h to hist; returns true in every thread of the block that finished last
-__device__ bool radix_flush(const unsigned int* h, unsigned long long* hist, EnergyStats* s, bool* last) {
-  for (int i = threadIdx.x; i < RBINS; i += blockDim.x)
-    if (h[i]) atomicAdd(&hist[i], (unsigned long long)h[i]);
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) *last = atomicAdd(&s->ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (*last) __threadfence();
-  return *last;
-}
-
-__global__ void __launch_bounds__(RH_T) k_stats_hist0(const double* __restrict__ e, size_t n, EnergyStats* s, int force,
-                                                     unsigned long long* hist) {
-  __shared__ unsigned int h[RBINS];
-  __shared__ long long wsum[RH_T / 32];
-  __shared__ double rlo[RH_T / 32], rhi[RH_T / 32];
-  __shared__ int rnan[RH_T / 32];
-  __shared__ bool last;
-  for (int i = threadIdx.x; i < RBINS; i += blockDim.x) h[i] = 0;
-  __syncthreads();
-  double lo = DBL_MAX, hi = -DBL_MAX;
-  int anynan = 0;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double v = e[i];
-    if (v != v) anynan = 1;
-    else { lo = fmin(lo, v); hi = fmax(hi, v); }
-    atomicAdd(&h[okey(v) >> (64 - RBITS)], 1u);
+  for (int u = 0; u < MED_E; u++) v[u] = i0 + u * step < n ? e[i0 + u * step] : 0.0;
+  auto each = [&](auto f) {
+#pragma unroll
+    for (int u = 0; u < MED_E; u++)
+      if (i0 + u * step < n) f(v[u], i0 + u * step);
+    for (size_t i = i0 + MED_E * step; i < n; i += 4 * step) {
+      double w[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) w[u] = i + u * step < n ? e[i + u * step] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (i + u * step < n) f(w[u], i + u * step);
+    }
+  };
+  // 1. the range of the energies
+  {
+    unsigned long long lo = ~0ull, hi = 0;
+    bool nan = false;
+    each([&](double x, size_t) {
+      if (x != x) {
+        nan = true;
+      } else {
+        const unsigned long long k = okey(x);
+        lo = k < lo ? k : lo;
+        hi = k > hi ? k : hi;
+      }
+    });
+    __syncwarp();
+    energy_range(&P, lo, hi, nan);
+    if (!grid_meet(s, &P, ++round)) return;
   }
-  for (int o = 16; o; o >>= 1) {
-    lo = fmin(lo, __shfl_xor_sync(0xffffffff, lo, o));
-    hi = fmax(hi, __shfl_xor_sync(0xffffffff, hi, o));
-    anynan |= __shfl_xor_sync(0xffffffff, anynan, o);
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { rlo[wid] = lo; rhi[wid] = hi; rnan[wid] = anynan; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < RH_T / 32; w++) { lo = fmin(lo, rlo[w]); hi = fmax(hi, rhi[w]); anynan |= rnan[w]; }
-    atomic_min_d(&s->lo, lo);
-    atomic_max_d(&s->hi, hi);
-    if (anynan) atomicOr(&s->nan, 1);
-  }
-  if (!radix_flush(h, hist, s, &last)) return;
+  const unsigned long long klo = __ldcg(&P.lo), khi = __ldcg(&P.hi);
+  const bool nan = __ldcg(&P.nan) != 0;
   // the reset needs the median unless every energy is above 1e-9 max + 1e-30 (phaseflow.rs:846-854)
-  const int snan = __ldcg(&s->nan);
-  const double slo = __ldcg(&s->lo), shi = __ldcg(&s->hi);
-  const bool skip = !snan && shi <= DBL_MAX / 2 && slo > 1e-9 * shi + 1e-30;
-  const bool need = force || !skip;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s->skip_reset = skip ? 1 : 0;
-    s->need_median = need ? 1 : 0;
-    s->median = snan ? nan("") : 0.0;
-  }
-  if (need && !snan) {
-    radix_pick(hist, s, 64 - RBITS, wsum);
-  } else {
-    for (int i = threadIdx.x; i < RBINS; i += blockDim.x) hist[i] = 0;
-    if (threadIdx.x == 0) s->ticket = 0;
-  }
-}
-
-// One pass over the elements that match the prefix: a block histogram of the digit, added to hist; the last block
-// picks.
-__global__ void __launch_bounds__(RH_T) k_radix_hist(const double* __restrict__ e, size_t n, EnergyStats* s, int pass,
-                                                    unsigned long long* hist) {
-  if (!s->need_median || s->nan) return;
-  __shared__ unsigned int h[RBINS];
-  __shared__ long long wsum[RH_T / 32];
-  __shared__ bool last;
-  for (int i = threadIdx.x; i < RBINS; i += blockDim.x) h[i] = 0;
-  __syncthreads();
-  int shift, bits;
-  digit_of(pass, shift, bits);
-  const unsigned long long prefix = s->prefix;
-  const int hib = 64 - RBITS * pass;  // bits already fixed above `hib`
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    unsigned long long k = okey(e[i]);
-    bool match = hib == 64 ? true : ((k >> hib) == (prefix >> hib));
-    if (match) atomicAdd(&h[(k >> shift) & ((1ULL << bits) - 1)], 1u);
-  }
-  __syncthreads();
-  if (!radix_flush(h, hist, s, &last)) return;
-  radix_pick(hist, s, shift, wsum);
-}
-
-constexpr int CBITS = 64 - 2 * RBITS;  // key bits below the bucket of the first two passes
-
-__global__ void k_radix_compact(const double* __restrict__ e, size_t n, EnergyStats* s, unsigned long long* cand) {
-  if (!s->need_median || s->nan) return;
-  const unsigned long long pre = s->prefix >> CBITS;
-  unsigned long long below = 0;
-  const int lane = threadIdx.x & 31;
-  for (size_t i0 = blockIdx.x * (size_t)blockDim.x; i0 < n; i0 += (size_t)gridDim.x * blockDim.x) {
-    const size_t i = i0 + threadIdx.x;
-    unsigned long long k = 0;
-    bool in = false;
-    if (i < n) {
-      k = okey(e[i]);
-      const unsigned long long kk = k >> CBITS;
-      in = kk == pre;
-      if (kk < pre && k > below) below = k;
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, in);
-    if (m) {  // one atomic per warp: the warp's matches take consecutive slots
-      unsigned base = 0;
-      if (lane == __ffs(m) - 1) base = atomicAdd(&s->ncand, (unsigned)__popc(m));
-      base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
-      const unsigned slot = base + __popc(m & ((1u << lane) - 1));
-      if (in) cand[slot] = k;  // slots < n: at most n elements match
-    }
-  }
-  for (int o = 16; o; o >>= 1) {
-    const unsigned long long v = __shfl_xor_sync(0xffffffffu, below, o);
-    below = v > below ? v : below;
-  }
-  if (lane == 0 && below) atomicMax(&s->below_max, below);
-}
-
-// the remaining CBITS bits of the median's key over the candidates (10-bit digits), and the largest key below it
-// after the passes: prefix = key of the element of rank n/2; for even n the one of rank n/2 - 1 is the same value
-// when `less` (elements below it) < n/2, else the largest element below it (lo_val)
-__device__ void median_finish(EnergyStats* s, size_t n) {
-  const double hi = okey_inv(s->prefix);
-  if (n % 2) {
-    s->median = hi;
-    return;
-  }
-  double lo = hi;
-  if (s->less >= (long long)(n / 2)) {
-    unsigned long long k = *(unsigned long long*)&s->lo_val;
-    lo = okey_inv(k);
-  }
-  s->median = (lo + hi) / 2.0;
-}
-
-// the last bits of the select over the candidates, then the median itself (thread 0)
-__global__ void __launch_bounds__(1024) k_radix_final(EnergyStats* s, const unsigned long long* __restrict__ cand,
-                                                      size_t n) {
-  if (!s->need_median) return;
-  if (s->nan) {
-    if (threadIdx.x == 0) s->median = nan("");
-    return;
-  }
-  const unsigned nc = s->ncand;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  __shared__ unsigned int h[1024];
-  __shared__ unsigned int wtot[32];
-  __shared__ unsigned long long sh_prefix, wmax[32];
-  __shared__ long long sh_rank, sh_less;
-  unsigned long long prefix = s->prefix;
-  long long rank = s->rank, less = s->less;
-  for (int shift = CBITS - 10; shift >= 0; shift -= 10) {
-    h[tid] = 0;
+  const double vlo = okey_inv(klo), vhi = okey_inv(khi);
+  const bool skip = !nan && vhi <= DBL_MAX / 2 && vlo > 1e-9 * vhi + 1e-30;
+  if (!force && skip) return;
+  double med = ::nan("");
+  if (!nan) {
+    // 2. the part of the range that holds the element of rank n / 2
+    const unsigned long long range = khi - klo;
+    const int bits = 64 - __clzll((long long)range), shift = bits > 12 ? bits - 12 : 0;
+    for (int i = tid; i < MED_BINS; i += MED_T) h[i] = 0;
     __syncthreads();
-    for (unsigned i = tid; i < nc; i += 1024) {
-      const unsigned long long k = cand[i];
-      if ((k >> (shift + 10)) == (prefix >> (shift + 10))) atomicAdd(&h[(k >> shift) & 1023], 1u);
-    }
+    each([&](double x, size_t) { atomicAdd(&h[(okey(x) - klo) >> shift], 1u); });
     __syncthreads();
-    const unsigned c = h[tid];
-    unsigned inc = c;
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned v = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += v;
+    for (int i = tid; i < MED_BINS; i += MED_T)
+      if (h[i]) atomicAdd(&hist[i], h[i]);
+    if (!grid_meet(s, &P, ++round)) {
+      if (i0 == 0) s->median = med;
+      return;
     }
-    if (lane == 31) wtot[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-      unsigned w = wtot[lane];
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += v;
+    long long rank = (long long)(n / 2), less = 0, before;
+    int bin;
+    block_pick([&](int i) { return __ldcg(hist + i); }, rank, bin, before);
+    rank -= before;
+    less += before;
+    // 3. that part's elements, and the largest key below it
+    const unsigned long long base = klo + ((unsigned long long)bin << shift);
+    const unsigned long long width = 1ull << shift;  // keys of the part: [base, base + width)
+    unsigned long long below = 0;
+    each([&](double x, size_t) {
+      const unsigned long long k = okey(x);
+      if (k < base) below = k > below ? k : below;
+      else if (k - base < width) cand[atomicAdd(&P.ncand, 1u)] = k;  // the active lanes' additions are made as one
+    });
+    __syncwarp();
+    for (int o = 16; o; o >>= 1) {
+      const unsigned long long v = __shfl_xor_sync(0xffffffffu, below, o);
+      below = v > below ? v : below;
+    }
+    if (lane == 0 && below > __ldcg(&P.below)) atomicMax(&P.below, below);
+    if (!grid_meet(s, &P, ++round)) {
+      if (i0 == 0) s->median = med;
+      return;
+    }
+    // 4. the element of that rank among the candidates
+    const unsigned nc = __ldcg(&P.ncand);
+    if (tid == 0) sh_below = __ldcg(&P.below);
+    if (nc <= MED_T) {
+      const unsigned long long key = (unsigned)tid < nc ? __ldcg(cand + tid) : ~0ull;
+      keys[tid] = key;
+      __syncthreads();
+      if ((unsigned)tid < nc) {
+        unsigned lt = 0, le = 0;
+        for (unsigned i = 0; i < nc; i++) {
+          lt += keys[i] < key;
+          le += keys[i] <= key;
+        }
+        if ((long long)lt <= rank && rank < (long long)le) {  // the equal keys of that rank write the same values
+          sh_key = key;
+          sh_less = less + lt;
+        }
       }
-      wtot[lane] = w;
+      __syncthreads();
+    } else {
+      unsigned long long prefix = 0;  // the digits fixed so far of key - base
+      for (int rem = shift; rem > 0;) {
+        const int d = rem < 12 ? rem : 12, sh = rem - d;
+        for (int i = tid; i < MED_BINS; i += MED_T) h[i] = 0;
+        __syncthreads();
+        for (unsigned i = tid; i < nc; i += MED_T) {
+          const unsigned long long k = __ldcg(cand + i) - base;
+          if ((k >> rem) == prefix) atomicAdd(&h[(k >> sh) & ((1u << d) - 1)], 1u);
+        }
+        __syncthreads();
+        block_pick([&](int i) { return h[i]; }, rank, bin, before);
+        rank -= before;
+        less += before;
+        prefix = (prefix << d) | (unsigned)bin;
+        rem = sh;
+      }
+      if (tid == 0) {
+        sh_key = base + prefix;
+        sh_less = less;
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    const long long excl = (long long)(inc - c) + (wid ? wtot[wid - 1] : 0);
-    if (excl <= rank && rank < excl + (long long)c) {  // exactly one thread
-      sh_prefix = prefix | ((unsigned long long)tid << shift);
-      sh_rank = rank - excl;
-      sh_less = less + excl;
+    const unsigned long long kmed = sh_key;
+    med = okey_inv(kmed);
+    // an even count's lower middle: the same value unless exactly n / 2 elements are below it, then the largest of those
+    if (n % 2 == 0 && sh_less >= (long long)(n / 2)) {
+      unsigned long long best = 0;
+      for (unsigned i = tid; i < nc; i += MED_T) {
+        const unsigned long long k = __ldcg(cand + i);
+        if (k < kmed && k > best) best = k;
+      }
+      for (int o = 16; o; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, best, o);
+        best = v > best ? v : best;
+      }
+      if (lane == 0 && best) atomicMax(&sh_below, best);
+      __syncthreads();
+      med = (okey_inv(sh_below) + med) / 2.0;
     }
-    __syncthreads();
-    prefix = sh_prefix;
-    rank = sh_rank;
-    less = sh_less;
   }
-  unsigned long long best = 0;
-  for (unsigned i = tid; i < nc; i += 1024) {
-    const unsigned long long k = cand[i];
-    if (k < prefix && k > best) best = k;
-  }
-  for (int o = 16; o; o >>= 1) {
-    const unsigned long long v = __shfl_xor_sync(0xffffffffu, best, o);
-    best = v > best ? v : best;
-  }
-  if (lane == 0) wmax[wid] = best;
-  __syncthreads();
-  if (tid == 0) {
-    best = s->below_max;
-    for (int w = 0; w < 32; w++) best = wmax[w] > best ? wmax[w] : best;
-    s->prefix = prefix;
-    s->rank = rank;
-    s->less = less;
-    *(unsigned long long*)&s->lo_val = best;
-    median_finish(s, n);
-  }
-}
-
-void launch_energy_median(const double* energy, size_t n, EnergyStats* stats, bool force_median,
-                          unsigned long long* scratch, cudaStream_t st, bool primed) {
-  unsigned long long* hist = scratch;
-  unsigned long long* cand = scratch + RBINS;
-  if (!primed) OFC_LAUNCH(k_stats_init, 1, 1, 0, st, stats, n);
-  OFC_LAUNCH(k_stats_hist0, 296, RH_T, 0, st, energy, n, stats, force_median ? 1 : 0, hist);
-  OFC_LAUNCH(k_radix_hist, 296, RH_T, 0, st, energy, n, stats, 1, hist);
-  OFC_LAUNCH(k_radix_compact, 296, 256, 0, st, energy, n, stats, cand);
-  OFC_LAUNCH(k_radix_final, 1, 1024, 0, st, stats, cand, n);
-}
-
-__global__ void k_reset(const double* __restrict__ energy, const double* __restrict__ uxin,
-                        const double* __restrict__ uyin, int n, EnergyStats* s, double* ux, double* uy,
-                        double* resid, double* slope, int prime) {
-  // the next median's start state, in place of its own k_stats_init launch (this kernel is the last reader of the
-  // select state's result, and it reads only median and skip_reset)
-  if (prime && blockIdx.x == 0 && threadIdx.x == 0) stats_prime(s, (size_t)n);
-  if (s->skip_reset) return;
-  const double thr = 1e-9 * s->median + 1e-30;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-    if (!(energy[p] > thr)) {
+  if (i0 == 0) s->median = med;
+  if (skip || !ux) return;
+  const double thr = 1e-9 * med + 1e-30;
+  each([&](double x, size_t p) {
+    if (!(x > thr)) {
       ux[p] = uxin[p];
       uy[p] = uyin[p];
       resid[p] = PI;
       for (int i = 0; i < 4; i++) slope[(size_t)i * n + p] = 0.0;
     }
-  }
+  });
 }
 
-void launch_reset(const double* energy, const double* ux_in, const double* uy_in, int n, EnergyStats* stats,
-                  double* ux, double* uy, double* resid, double* slope, cudaStream_t st, bool prime_next) {
-  OFC_LAUNCH(k_reset, div_up(n, 256), 256, 0, st, energy, ux_in, uy_in, n, stats, ux, uy, resid, slope,
-             prime_next ? 1 : 0);
+void launch_energy_stats_init(EnergyStats* stats, unsigned long long* scratch, cudaStream_t st) {
+  OFC_CUDA(cudaMemsetAsync(scratch, 0, 2 * MED_BINS * sizeof(unsigned), st));
+  OFC_LAUNCH(k_stats_init, 1, 1, 0, st, stats);
+}
+
+void launch_median_reset(const double* energy, size_t n, EnergyStats* stats, int half, bool force,
+                         unsigned long long* scratch, const double* ux_in, const double* uy_in, double* ux, double* uy,
+                         double* resid, double* slope, cudaStream_t st) {
+  int dev = 0, sms = 0;
+  OFC_CUDA(cudaGetDevice(&dev));
+  OFC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // one block per SM at most: every block is resident in a cooperative launch
+  const int grid = (int)std::min<size_t>((size_t)sms, std::max<size_t>(1, n / MED_PER));
+  unsigned* hist = (unsigned*)scratch;
+  unsigned long long* cand = scratch + MED_BINS;  // after the two histograms
+  int f = force;
+  void* args[] = {&energy, &n, &stats, &half, &f, &hist, &cand, &ux_in, &uy_in, &ux, &uy, &resid, &slope};
+  void* tok = nullptr;
+  if (g_profiler) prof_before("k_median_reset", st, &tok);
+  OFC_CUDA(cudaLaunchCooperativeKernel((const void*)k_median_reset, dim3(grid), dim3(MED_T), args, 0, st));
+  if (tok) prof_after(tok, st);
+  if (g_launch_counter) ++*g_launch_counter;
 }
 
 // ---------------------------------------------------------------- confidence

@@ -57,33 +57,29 @@ void launch_moments_solve(const double* sums, const double* ux, const double* uy
                           const double* mtaps, int r, const MomTaps& tp, double* yplanes, double* oux, double* ouy,
                           double* energy, double* resid, double* slope, cudaStream_t st);
 
-// min / max / NaN of the energy and whether its median is needed (stats: device struct, see fine.cu)
+// The state of the energy medians of a refinement (device). Two halves alternate: a median uses one and clears the other
+// for the next.
 struct EnergyStats {
-  double lo, hi;
-  int nan;
-  int need_median;  // set by the reduction: the reset needs it, or the caller forces it
-  int skip_reset;   // every energy is above 1e-9 max + 1e-30: no pixel is reset
   double median;
-  // radix-select state
-  unsigned long long prefix;
-  long long rank;
-  long long less;
-  double lo_val;
-  unsigned int ticket;  // blocks of the current histogram pass that are done (the last one picks)
-  unsigned int ncand;   // elements in the bucket of the first two digits (candidates of the final select)
-  unsigned long long below_max;  // the largest key below that bucket
+  unsigned timeouts;  // grid barriers that gave up (the median is NaN then)
+  struct Half {
+    unsigned long long lo, hi;  // the smallest and largest energy as order-preserving keys (~0 and 0: none yet)
+    unsigned long long below;   // the largest key below the median's bucket
+    unsigned nan;               // an energy is NaN
+    unsigned ncand;             // elements in the median's bucket
+    unsigned bar;               // arrivals at the grid barriers
+  } half[2];
 };
-// unsigned long long of the median's scratch for n energies: the histogram, then up to n candidates
+// unsigned long long of the median's scratch for n energies: two histograms of 4096 counts, then up to n candidates
 inline size_t median_scratch(size_t n) { return 4096 + n; }
-// stats->lo/hi/nan/skip_reset of energy, and its median into stats->median (np.median) when the reset needs it
-// or force_median; scratch: median_scratch(n) unsigned long long whose first 4096 are zero (they are left zero)
-// primed: stats already hold a median's start state (a launch_reset with prime_next since the last median)
-void launch_energy_median(const double* energy, size_t n, EnergyStats* stats, bool force_median,
-                          unsigned long long* scratch, cudaStream_t st, bool primed = false);
-// reset below 1e-9 median + 1e-30 (phaseflow.py:149-151,158-161); prime_next: also put the next median's start state
-// into stats (its median and skip_reset stay as they are)
-void launch_reset(const double* energy, const double* ux_in, const double* uy_in, int n, EnergyStats* stats,
-                  double* ux, double* uy, double* resid, double* slope, cudaStream_t st, bool prime_next = false);
+// the start state of both halves and zero histograms
+void launch_energy_stats_init(EnergyStats* stats, unsigned long long* scratch, cudaStream_t st);
+// The reset below 1e-9 median + 1e-30 (phaseflow.py:149-151,158-161) of ux, uy, resid and slope (ux null: no reset) when an
+// energy needs it, and the median into stats->median (np.median) when the reset needs it or `force`, in one launch on
+// `half` of the state
+void launch_median_reset(const double* energy, size_t n, EnergyStats* stats, int half, bool force,
+                         unsigned long long* scratch, const double* ux_in, const double* uy_in, double* ux, double* uy,
+                         double* resid, double* slope, cudaStream_t st);
 
 // confidence before the border rule (phaseflow.py:320-323) and low = conf < conf_min; with border = true
 // also the border rule (phaseflow.py:297-317,508-510): conf_out (f32), low (u8), conf64 (nullable)

@@ -228,6 +228,21 @@ def test_median(T):
     assert T.median(v) == np.median(v)
 
 
+@pytest.mark.parametrize("n", [1, 2, 1023, 1024, 1025, 8191, 8192, 16384, 16385, 148 * 8192 + 3, 3_000_000])
+def test_median_blocks_and_special_values(T, n):
+    """The cooperative median at the edges of its blocks (8192 energies a block up to one block per SM, then more per
+    thread) against np.median exactly: spread values, one value throughout, infinities, subnormals, a NaN."""
+    rng = np.random.default_rng(n)
+    for v in (rng.exponential(size=n), np.full(n, 0.25), rng.standard_normal(n) * 10.0 ** rng.integers(-300, 300, n),
+              rng.integers(0, 3, n).astype(np.float64), rng.random(n) * 1e-310):
+        assert T.median(v) == np.median(v)
+    v = rng.exponential(size=n)
+    v[: n // 3] = np.inf
+    assert T.median(v) == np.median(v)
+    v[n // 2] = np.nan
+    assert np.isnan(T.median(v))
+
+
 def test_large_components(T, oracle):
     rng = np.random.default_rng(9)
     for p in (0.3, 0.5, 0.6):
