@@ -3,8 +3,8 @@
 // One thread block transforms C interleaved lines held in shared memory (element i of line l at
 // buf[i * C + l]), ping-ponging between two buffers of L * C values: each Stockham stage reads a butterfly's
 // inputs from one and writes its outputs to the other. Radices 2, 4 and 8 have register butterflies, 3, 5, 7,
-// 11 and 13 the symmetric odd form, other primes (up to 31) a direct DFT. Twiddles come from a table rounded
-// from float64.
+// 11, 13, 17 and 19 the symmetric odd form, 23, 29 and 31 a direct DFT. Twiddles come from a table rounded from
+// float64.
 //
 // The pass structure of one "responses" evaluation (per outer iteration of the fine stage):
 //   rows:    reflect pad + real->complex + forward row FFT                      (read 4 B/px, write 8 B/px)
@@ -248,24 +248,33 @@ std::vector<float2> fft_twiddles(int L) {
   return t;
 }
 
-// threads of a block of a runtime plan: the count up to RT_T for which the stages' rounds of butterflies (weighted by
-// the butterfly's length) leave the fewest threads idle
-static int rt_threads(const FftPlan& pl, int C) {
+// Threads of a block of a runtime plan that holds `smem` bytes: the count whose blocks finish most lines per time on an SM.
+// A block's line takes the longer of its latency (the rounds of butterflies of its stages one after the other, an
+// instruction of a lone warp every 6 cycles, a barrier per stage) and its share of the issue slots (2.4 instructions per
+// cycle between the resident blocks, as many as shared memory and 80 registers per thread admit). Small transforms get
+// several blocks of few threads with little idling in the stages of large radices, a transform that fills shared memory
+// by itself many threads (Bluestein's 4096 on a column pair: one block per SM). *cycles: that time per block.
+static int rt_threads(const FftPlan& pl, int C, size_t smem, double* cycles = nullptr) {
   const int SL = fft_work_len(pl);
-  int best = RT_T;
-  double bc = 1e30;
+  const int fit = std::max<int>(1, (int)((227 * 1024) / (smem + 1024)));
+  int best = 256;
+  double bt = 1e300;
   for (int T = 96; T <= RT_T; T += 32) {
-    double c = 0;
+    const int blocks = std::min(fit, std::max(1, 65536 / (80 * T)));
+    double lat = 0, work = 0;
     for (int i = 0; i < pl.nst; i++) {
-      const int nb = SL / pl.p[i] * C, rounds = (nb + T - 1) / T;
-      c += (double)rounds * (pl.p[i] * pl.p[i] / 2 + 16 * pl.p[i]);
+      const int P = pl.p[i], sh = P >= 23 ? 4 : 1, nb = sh > 1 ? (SL / P * C + 31) / 32 * 32 * sh : SL / P * C;
+      const double c = sh > 1 ? 4.5 * P * P / sh + 30.0 * P : (P % 2 ? (P - 1) * (P - 1) : 8 * P) + 25.0 * P;  // instructions
+      lat += (double)((nb + T - 1) / T) * c * 6.0 + 150.0;
+      work += (double)nb / 32.0 * c;
     }
-    c *= T + 32;  // more threads per block, fewer blocks per SM
-    if (c < bc * 0.999) {
-      bc = c;
+    const double t = std::max(lat / blocks, work / 2.4);
+    if (t < bt * 0.995) {
+      bt = t;
       best = T;
     }
   }
+  if (cycles) *cycles = bt;
   return best;
 }
 
@@ -466,6 +475,30 @@ __device__ __forceinline__ void odd_butterfly(Load in, bool inv, Emit emit) {
 constexpr int FFT_PAD = 4;
 __host__ __device__ constexpr int fft_buf_len(int L, int C) { return L * C + ((L * C) >> FFT_PAD) + 1; }
 
+// w_P^(j k) = exp(-2 pi i j k / P) of the direct DFTs (P = 23, 29, 31), row k: read uniformly by a warp, from constant memory
+template <int P>
+struct DirectCoef {
+  float2 w[P * P] = {};
+  constexpr DirectCoef() {
+    for (int k = 0; k < P; k++)
+      for (int j = 0; j < P; j++) {
+        double c = 0, s = 0;
+        ct_sincos((j * k) % P, P, c, s);
+        w[k * P + j].x = (float)c;
+        w[k * P + j].y = (float)(-s);
+      }
+  }
+};
+__constant__ DirectCoef<23> c_direct23{};
+__constant__ DirectCoef<29> c_direct29{};
+__constant__ DirectCoef<31> c_direct31{};
+template <int P>
+__device__ __forceinline__ const float2* direct_coef() {
+  if constexpr (P == 23) return c_direct23.w;
+  else if constexpr (P == 29) return c_direct29.w;
+  else return c_direct31.w;
+}
+
 // Shared memory by 32-bit addresses: the stages are functions of their own, and through a generic pointer each of their
 // accesses would cost 64-bit address arithmetic and the generic path.
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -478,10 +511,12 @@ __device__ __forceinline__ void sts2(unsigned a, float2 v) {
   asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
 }
 
-// The butterfly of radix P (P = 0: a direct DFT of runtime radix RP) on inputs in(j), j < P, with outputs
-// through emit(k, value) (which applies the inter-stage twiddle); tw_m(m) = w_P^m for the direct DFT.
-template <int P, class C2, class In, class Emit, class TwM>
-__device__ __forceinline__ void butterfly(In in, Emit emit, TwM tw_m, int RP, bool inv) {
+// threads that share a butterfly's outputs: the direct sums' (a line of 841 = 29 29 has 29 butterflies per stage)
+__host__ __device__ constexpr int butterfly_share(int P) { return P >= 23 ? 4 : 1; }
+// The butterfly of radix P on inputs in(j), j < P, with outputs through emit(k, value) (which applies the inter-stage
+// twiddle); part: which of butterfly_share(P) parts of the outputs.
+template <int P, class C2, class In, class Emit>
+__device__ __forceinline__ void butterfly(In in, Emit emit, bool inv, int part = 0) {
   if constexpr (P == 2) {
     C2 a0 = in(0), a1 = in(1);
     emit(0, cadd(a0, a1));
@@ -525,27 +560,42 @@ __device__ __forceinline__ void butterfly(In in, Emit emit, TwM tw_m, int RP, bo
     emit(7, csub(e[3], t3));
   } else if constexpr (P == 3 || P == 5 || P == 7 || P == 11 || P == 13 || P == 17 || P == 19) {
     odd_butterfly<P, C2>(in, inv, emit);
-  } else {
-    for (int k = 0; k < RP; k++) {
-      C2 acc = in(0);
-      int jk = 0;
-      for (int j = 1; j < RP; j++) {
-        jk += k;
-        if (jk >= RP) jk -= RP;
-        C2 av = in(j);
-        C2 w = tw_m(jk);
-        acc.x = fma(av.x, w.x, fma(-av.y, w.y, acc.x));
-        acc.y = fma(av.x, w.y, fma(av.y, w.x, acc.y));
+  } else {  // the direct sum, inputs in registers, two outputs at a time; the inverse as conj(forward(conj))
+    static_assert(P == 23 || P == 29 || P == 31, "a radix with a butterfly");
+    C2 v[P];
+#pragma unroll
+    for (int j = 0; j < P; j++) {
+      v[j] = in(j);
+      if (inv) v[j].y = -v[j].y;
+    }
+    const float2* W = direct_coef<P>();
+#pragma unroll 1
+    for (int k = 2 * part; k < P; k += 2 * butterfly_share(P)) {
+      const float2 *w0 = W + k * P, *w1 = W + (k + 1 < P ? k + 1 : k) * P;
+      C2 a = v[0], b = v[0];
+#pragma unroll
+      for (int j = 1; j < P; j++) {
+        const float2 p = w0[j], q = w1[j];
+        a.x = fmaf(v[j].x, p.x, fmaf(-v[j].y, p.y, a.x));
+        a.y = fmaf(v[j].x, p.y, fmaf(v[j].y, p.x, a.y));
+        b.x = fmaf(v[j].x, q.x, fmaf(-v[j].y, q.y, b.x));
+        b.y = fmaf(v[j].x, q.y, fmaf(v[j].y, q.x, b.y));
       }
-      emit(k, acc);
+      if (inv) {
+        a.y = -a.y;
+        b.y = -b.y;
+      }
+      emit(k, a);
+      if (k + 1 < P) emit(k + 1, b);
     }
   }
 }
 
 // One Stockham stage of radix P from buffer A to buffer B; C interleaved lines of length L, C = 1 << LC. q of a butterfly
 // comes from a multiplication by a precomputed reciprocal (magic = ceil(2^32 / s), exact for the sizes here). Radices 2,
-// 4, 8 have hand-written butterflies, 3 ... 19 the symmetric odd form, and any other radix (P = 0 here) a direct DFT with
-// its inputs read from shared memory. Each radix is its own non-inlined function, so that the registers of one radix's
+// 4, 8 have hand-written butterflies, 3 ... 19 the symmetric odd form, 23, 29 and 31 the direct sum (its inputs in
+// registers, its coefficients in constant memory and four threads to a butterfly: rows of 841 = 29 29 take 0.42 ms per
+// launch of the row pass at 777 x 1500, 1.25 ms with the inputs read from shared memory for every output). Each radix is its own non-inlined function, so that the registers of one radix's
 // butterfly do not add to another's. Butterfly b reads elements b + j istep (b = bi C + l with bi = q s + r). ISH, OSH:
 // A, B in the padded layout (only a stage of an even radix with s C < 32 writes it: an odd radix's outputs fall on
 // distinct banks as they are). IN, OUT: what the first stage does to its inputs and the last to its outputs.
@@ -584,17 +634,19 @@ __device__ __forceinline__ float2 stage_in(unsigned a, int i, int lc, const Stag
 }
 
 template <int P, int LC, int IN, int OUT, bool ISH, bool OSH>
-__device__ __noinline__ void stage_loop(unsigned A, unsigned B, int Pr, int s, int m,
-                                        unsigned magic, const float2* __restrict__ stw, const float2* __restrict__ tw,
-                                        bool inv, StageEx ex) {
-  const int RP = P ? P : Pr;
+__device__ __noinline__ void stage_loop(unsigned A, unsigned B, int s, int m, unsigned magic,
+                                        const float2* __restrict__ stw, bool inv, StageEx ex) {
   constexpr int C = 1 << LC;
-  const int LP = s * m;  // L / RP
+  const int LP = s * m;  // L / P
   const int nb = LP << LC, istep = nb, ostep = s << LC;
-  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    const int l = b & (C - 1), bi = b >> LC;
+  // a shared butterfly's parts lie whole warps apart (a warp reads the coefficients uniformly)
+  constexpr int SH = butterfly_share(P);
+  const int nbw = SH > 1 ? (nb + 31) & ~31 : nb;
+  for (int t = threadIdx.x; t < nbw * SH; t += blockDim.x) {
+    const int part = SH > 1 ? t / nbw : 0, b = t - part * nbw, l = b & (C - 1), bi = b >> LC;
+    if (SH > 1 && b >= nb) continue;
     const int q = s == 1 ? bi : (m == 1 ? 0 : (int)__umulhi((unsigned)bi, magic));
-    const int ob = ((bi + (RP - 1) * q * s) << LC) + l;
+    const int ob = ((bi + (P - 1) * q * s) << LC) + l;
     auto in = [&](int j) {
       const int i = b + j * istep;
       return stage_in<IN>(A + 8u * (unsigned)(ISH ? i + (i >> FFT_PAD) : i), i, LC, ex);
@@ -612,11 +664,7 @@ __device__ __noinline__ void stage_loop(unsigned A, unsigned B, int Pr, int s, i
       }
       sts2(B + 8u * (unsigned)(OSH ? o + (o >> FFT_PAD) : o), val);
     };
-    auto tw_m = [&](int mm) {  // w_P^mm
-      const float2 w = __ldg(tw + (size_t)mm * LP);
-      return inv ? conjf2(w) : w;
-    };
-    butterfly<P, float2>(in, emit, tw_m, RP, inv);
+    butterfly<P, float2>(in, emit, inv, part);
   }
 }
 
@@ -625,9 +673,6 @@ __device__ __noinline__ void stage_loop(unsigned A, unsigned B, int Pr, int s, i
 // the transform's direction.
 template <int P, int S, int L, int C, int ISH, int OSH, int IN, int OUT>
 __device__ __noinline__ void stage_fixed(unsigned A, unsigned B, const float2* __restrict__ stw, bool inv, StageEx ex) {
-  constexpr int PB =
-      (P == 2 || P == 3 || P == 4 || P == 5 || P == 7 || P == 8 || P == 11 || P == 13 || P == 17 || P == 19) ? P : 0;
-  static_assert(PB != 0, "a plan of the radices with butterflies");
   constexpr int M = L / (P * S), NB = (L / P) * C, ISTEP = S * M * C, OSTEP = S * C, LC = C == 2 ? 1 : 0;
   static_assert(IN == IN_PLAIN || ISTEP % C == 0, "an element's column is the thread's");
   for (int b = threadIdx.x; b < NB; b += blockDim.x) {
@@ -651,8 +696,7 @@ __device__ __noinline__ void stage_fixed(unsigned A, unsigned B, const float2* _
       if constexpr (OSH < 31) sts2(B + 8u * (unsigned)(o + (o >> OSH)), val);
       else sts2(B + 8u * (unsigned)o, val);
     };
-    auto tw_m = [&](int) { return make_float2(0.f, 0.f); };  // the direct DFT's, not reached
-    butterfly<PB, float2>(in, emit, tw_m, P, inv);
+    butterfly<P, float2>(in, emit, inv);
   }
 }
 
@@ -711,7 +755,7 @@ __device__ __forceinline__ bool fft_stage(const float2* A, float2* B, const FftP
     constexpr bool EVEN = PP == 2 || PP == 4 || PP == 8;
     auto call = [&](auto ic, auto oc) {
       constexpr bool IS = decltype(ic)::value && IN == IN_PLAIN, OS = decltype(oc)::value && EVEN && OUT == OUT_PLAIN;
-      stage_loop<PP, LC, IN, OUT, IS, OS>(smem_addr(A), smem_addr(B), P, s, m, pl.magic[st], pl.stw + pl.so[st] + (inv ? pl.nstw : 0), pl.tw, inv, ex);
+      stage_loop<PP, LC, IN, OUT, IS, OS>(smem_addr(A), smem_addr(B), s, m, pl.magic[st], pl.stw + pl.so[st] + (inv ? pl.nstw : 0), inv, ex);
     };
     if (ish) {
       if (EVEN && osh) call(std::true_type{}, std::true_type{});
@@ -733,7 +777,9 @@ __device__ __forceinline__ bool fft_stage(const float2* A, float2* B, const FftP
     case 13: go(integral_constant<int, 13>{}); break;
     case 17: go(integral_constant<int, 17>{}); break;
     case 19: go(integral_constant<int, 19>{}); break;
-    default: go(integral_constant<int, 0>{}); break;
+    case 23: go(integral_constant<int, 23>{}); break;
+    case 29: go(integral_constant<int, 29>{}); break;
+    default: go(integral_constant<int, 31>{}); break;
   }
   __syncthreads();
   return osh;
@@ -926,9 +972,8 @@ __device__ __forceinline__ int reflect_near(int i, int n) {
 // 2112 = 8 8 3 11; the plan fixed at compile time), and FIXL = -FFT_FIXED_M (Bluestein with that inner length fixed);
 // the launchers pick by the plan.
 
-// blocks per SM of the runtime plans' kernels (80 registers; two blocks at 128 registers took 0.472 ms, four at 64 0.60 ms
-// in the row pass below)
-constexpr int RT_MINB = 3;
+// the runtime plans' kernels keep to 80 registers (at 128 registers the row pass below took 0.472 ms, at 64 0.60 ms)
+constexpr int RT_MINB = 1;
 // buffer stride of the kernels that stage several lines: fft_buf_len rounded up to an even count (16-byte aligned)
 __host__ __device__ constexpr int fft_buf_stride(int L, int C) { return (fft_buf_len(L, C) + 1) & ~1; }
 
@@ -956,7 +1001,7 @@ __global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? FFT_TMAX : RT_T, FIXL 
 constexpr int COLS_TMAX = 320;  // threads per block of the split column pass
 
 template <int C, int FIXL>
-__global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? COLS_TMAX : RT_T, 3) k_fft_cols_fwd(const float2* Tin, FftPlan plh, int pw, float2* S) {
+__global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? COLS_TMAX : RT_T, FIXL > 0 || FIXL < -1 ? 3 : RT_MINB) k_fft_cols_fwd(const float2* Tin, FftPlan plh, int pw, float2* S) {
   constexpr int LC = C == 4 ? 2 : (C == 2 ? 1 : 0);
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* A = (float2*)smraw;
@@ -989,48 +1034,49 @@ __global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? COLS_TMAX : RT_T, 3) k
 
 // The inverse column pass with the spectrum of a column pair staged once per block: the block copies its two
 // columns of S (ph x 2) into shared memory, then for each of its planes multiplies them by the plane's factor into
-// A, inverts along y (A, B) and stores the pair. REFPACK = false: the responses of the filters
-// [RESP_G blockIdx.y, RESP_G (blockIdx.y + 1)) (x G_k and the B-spline prefilter's periodic factors, inverse,
+// A, inverts along y (A, B) and stores the pair. REFPACK = false: the responses of the k1 filters
+// [k1 blockIdx.y, k1 (blockIdx.y + 1)) (x G_k and the B-spline prefilter's periodic factors, inverse,
 // the prefilter's edge terms along y) into plane k of U. REFPACK = true: variant v = blockIdx.y of the reference
 // pack (S G, S G i fx, S G i fy; factors in float64) of the filters [k0, k1) into plane 3 (k - k0) + v of U.
-// A thread's column is fixed (blockDim is even), so the x factors are read once.
-constexpr int RESP_G = 4;
+// A thread's column is fixed (blockDim is even), so the x factors are read once. C = 1: a single column per block, for
+// Bluestein plans whose pair would leave an SM's shared memory room for too few blocks.
 
 // threads of the fixed-length column-pair kernel: the responses COLS_TMAX; the reference pack, whose float64 factors
 // take more time per element, one per radix-8 butterfly of the two columns (2 x 2112 / 8)
 constexpr int PAIR_T_REF = 544;
 template <bool REFPACK>
 constexpr int pair_threads(int fixl) { return fixl > 0 && REFPACK ? PAIR_T_REF : (fixl == 0 || fixl == -1 ? RT_T : COLS_TMAX); }
-template <bool REFPACK, int FIXL>
+template <bool REFPACK, int FIXL, int C>
 __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), FIXL == 0 || FIXL == -1 ? RT_MINB : 2) k_fft_cols_pair(const float2* __restrict__ S, FftPlan plh, int pw,
                                                                 GaborTables g, int k0, int k1, float2* __restrict__ U) {
-  constexpr int C = 2;
+  static_assert(C == 2 || FIXL == -1, "one column per block: Bluestein's runtime plans");
+  constexpr int LC = C - 1;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ph = FIXL > 0 ? FIXL : plh.L, n = ph * C, tid = threadIdx.x, nt = blockDim.x;
   float2* raw = (float2*)smraw;
-  float2* A = raw + n;
+  float2* A = raw + ((n + 1) & ~1);
   float2* B = A + fft_buf_stride(FIXL > 0 ? FIXL : fft_work_len(plh), C);
   const int x0 = blockIdx.x * C;
-  const bool rows16 = x0 + 1 < pw && pw % 2 == 0;  // each row of the pair is 16 bytes on a 16-byte boundary
+  const bool rows16 = C == 2 && x0 + 1 < pw && pw % 2 == 0;  // each row of the pair is 16 bytes on a 16-byte boundary
   if (rows16) {
     for (int y = tid; y < ph; y += nt) __pipeline_memcpy_async(raw + 2 * y, S + (size_t)y * pw + x0, 16);
     __pipeline_commit();
     __pipeline_wait_prior(0);
   } else {
     for (int i = tid; i < n; i += nt) {
-      const int y = i >> 1, x = x0 + (i & 1);
+      const int y = i >> LC, x = x0 + (i & (C - 1));
       raw[i] = x < pw ? S[(size_t)y * pw + x] : make_float2(0.f, 0.f);
     }
   }
   __syncthreads();
-  const int x = min(x0 + (tid & 1), pw - 1);
+  const int x = min(x0 + (tid & (C - 1)), pw - 1);
   auto store = [&](const float2* r, int plane) {
     float2* dst = U + (size_t)plane * ph * pw + x0;
     if (rows16) {
       for (int y = tid; y < ph; y += nt) *(float4*)(dst + (size_t)y * pw) = *(const float4*)(r + 2 * y);
     } else {
       for (int i = tid; i < n; i += nt)
-        if (x0 + (i & 1) < pw) dst[(size_t)(i >> 1) * pw + (i & 1)] = r[i];
+        if (x0 + (i & (C - 1)) < pw) dst[(size_t)(i >> LC) * pw + (i & (C - 1))] = r[i];
     }
   };
   // the same with the prefilter's edge terms along y (constants kc of the two columns) added as the rows are stored
@@ -1045,13 +1091,14 @@ __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), FIXL == 0 || FIXL
       }
     } else {
       for (int i = tid; i < n; i += nt)
-        if (x0 + (i & 1) < pw) dst[(size_t)(i >> 1) * pw + (i & 1)] = bspline_edge_fix(r[i], i >> 1, ph, kc[i & 1]);
+        if (x0 + (i & (C - 1)) < pw)
+          dst[(size_t)(i >> LC) * pw + (i & (C - 1))] = bspline_edge_fix(r[i], i >> LC, ph, kc[i & (C - 1)]);
     }
   };
   if (!REFPACK) {
     const float hx = __ldg(g.hxf + x), omx = __ldg(g.omxf + x), bx = __ldg(g.bxf + x);
-    const int kend = min(g.F, (int)(blockIdx.y + 1) * RESP_G);
-    for (int k = blockIdx.y * RESP_G; k < kend; k++) {
+    const int kend = min(g.F, (int)(blockIdx.y + 1) * k1);
+    for (int k = blockIdx.y * k1; k < kend; k++) {
       // G = (hx + omx omy) ex ey (bx by): the x factors of the thread's column, (omy, ey by) from the row table
       const float exb = __ldg(g.exf + (size_t)k * pw + x) * bx;
       StageEx ex{};
@@ -1062,8 +1109,8 @@ __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), FIXL == 0 || FIXL
       float2* r;
       if constexpr (FIXL > 0) r = fft_run_fixed<FIXL, C, 0, IN_MUL, OUT_PLAIN>(raw, A, B, plh, true, ex);
       else if constexpr (FIXL < -1) r = fft_bluestein_fixed<-FIXL, C, IN_MUL>(raw, A, B, plh, true, ex);
-      else if constexpr (FIXL == 0) r = fft_stages<1, IN_MUL, OUT_PLAIN>(raw, A, B, nullptr, plh, ph, true, ex);
-      else r = fft_bluestein<1, IN_MUL>(raw, A, B, nullptr, plh, true, ex);
+      else if constexpr (FIXL == 0) r = fft_stages<LC, IN_MUL, OUT_PLAIN>(raw, A, B, nullptr, plh, ph, true, ex);
+      else r = fft_bluestein<LC, IN_MUL>(raw, A, B, nullptr, plh, true, ex);
       float2* idle = r == A ? B : A;
       bspline_edge_consts<C>(r, ph, (float4*)idle);  // the prefilter's edge terms along y, added by the store
       store_edges(r, (const float4*)idle, k);
@@ -1110,7 +1157,7 @@ __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), FIXL == 0 || FIXL
         }
       } else {
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
-          const int y = i >> 1;
+          const int y = i >> LC;
           mul(i, __ldg(g.omy + y), __ldg(eyk + y), v == 2 ? __ldg(g.fy + y) : 0.0);
         }
       }
@@ -1125,7 +1172,7 @@ __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), FIXL == 0 || FIXL
 // The same inverse column pass with one block per (C columns, plane) and no staged spectrum: the form for padded
 // heights whose column pair does not fit in shared memory beside the two transform buffers.
 template <int C, bool REFPACK, int FIXL>
-__global__ void __launch_bounds__(RT_T, 3) k_fft_cols_inv_filter(const float2* __restrict__ S, FftPlan plh, int pw,
+__global__ void __launch_bounds__(RT_T, RT_MINB) k_fft_cols_inv_filter(const float2* __restrict__ S, FftPlan plh, int pw,
                                                                       GaborTables g, int k0, float2* __restrict__ U) {
   constexpr int LC = C == 4 ? 2 : (C == 2 ? 1 : 0);
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1236,7 +1283,7 @@ __global__ void __launch_bounds__(FIXL > 0 ? 288 : FFT_TMAX, FIXL > 0 ? 3 : 2)
 // launch; 0.838 ms with the four buffers of M, uncoalesced twiddles and separate passes for the chirp and filter products):
 // a block takes one node row. The two raw lines keep buffers of L values and receive
 // their own results; only the two scratch buffers have the work length (Bluestein's M is about 2 L). More blocks fit per
-// SM than with four buffers of M and a prefetch of the next row, and blocks of at most RT_T threads (rt_threads) leave few
+// SM than with four buffers of M and a prefetch of the next row, and blocks of few threads (rt_threads) leave few
 // warps without a butterfly in the stages of large radices. Issue slots (55 %) and barriers bound it.
 template <int FIXL>
 __global__ void __launch_bounds__(RT_T, RT_MINB) k_fft_rows_inv_resp_rt(const float2* __restrict__ U, FftPlan plw, int ph, int F,
@@ -1336,7 +1383,7 @@ __global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? FFT_TMAX : RT_T, FIXL 
 }
 
 template <int FIXL>
-__global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? FFT_TMAX : RT_T, 2) k_fft_lines(float2* data, FftPlan pl, int inv) {
+__global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? FFT_TMAX : RT_T, FIXL > 0 || FIXL < -1 ? 2 : RT_MINB) k_fft_lines(float2* data, FftPlan pl, int inv) {
   extern __shared__ float2 sm[];
   const int L = FIXL > 0 ? FIXL : pl.L;
   float2* row = data + (size_t)blockIdx.x * L;
@@ -1361,10 +1408,10 @@ static size_t smem_prefilter(int L, int C, int T) {
   (void)T;
   return std::max<size_t>(2 * fbytes(L, C), fbytes(L, C) + 16 + (size_t)C * sizeof(float4));
 }
-// k_fft_cols_pair: the column pair (2 L values) and two buffers of the work length (L, or Bluestein's M) at the even
+// k_fft_cols_pair: the C columns (C L values) and two buffers of the work length (L, or Bluestein's M) at the even
 // stride
-static size_t smem_cols_pair(int L, int WL) {
-  return ((size_t)2 * L + 2 * (size_t)fft_buf_stride(WL, 2)) * sizeof(float2);
+static size_t smem_cols(int L, int WL, int C) {
+  return ((size_t)C * L + 1 + 2 * (size_t)fft_buf_stride(WL, C)) / 2 * 2 * sizeof(float2);
 }
 // k_fft_rows_inv_resp: four line buffers at the even stride
 static size_t smem_rows_resp(int L) { return 4 * (size_t)fft_buf_stride(L, 1) * sizeof(float2); }
@@ -1400,13 +1447,36 @@ bool fft_fixed_length(int L) {
   return L == 320 || L == 576 || L == 832 || L == 1024 || L == 1088 || L == 1600 || L == FFT_FIXED_L;
 }
 
-// blocks of a persistent launch: as many as are resident at once, at most one per unit of work
-static int persistent_blocks(const void* fn, int threads, size_t smem, int work) {
+// blocks of a kernel resident at once on the device
+static int resident_blocks(const void* fn, int threads, size_t smem) {
   int dev = 0, sms = 0, per = 0;
   OFC_CUDA(cudaGetDevice(&dev));
   OFC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   OFC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem));
-  return std::max(1, std::min(work, std::max(per, 1) * sms));
+  return std::max(per, 1) * sms;
+}
+
+// blocks of a persistent launch: as many as are resident at once, at most one per unit of work
+static int persistent_blocks(const void* fn, int threads, size_t smem, int work) {
+  return std::max(1, std::min(work, resident_blocks(fn, threads, smem)));
+}
+
+// The filters a block of the responses' column pass takes in turn from its staged column pair: the count whose waves of
+// `resident` blocks take the least time, a block's time being its filters plus 0.4 of one for the staging. Few columns
+// (small images) spread their filters over the chip, many stage their pair once for several; between them the count
+// that fills the last wave best.
+static int resp_group(int pairs, int F, int resident) {
+  int best = 1;
+  double bc = 1e30;
+  for (int G = 1; G <= std::min(F, 6); G++) {
+    const long blocks = (long)pairs * ((F + G - 1) / G);
+    const double c = (double)((blocks + resident - 1) / resident) * (G + 0.4);
+    if (c < bc * 0.999) {
+      bc = c;
+      best = G;
+    }
+  }
+  return best;
 }
 
 bool fft_fits(int ph, int pw) {
@@ -1425,8 +1495,8 @@ bool fft_fits(int ph, int pw) {
 static bool runtime_plan(const FftPlan& pl) { return pl.M ? pl.M != FFT_FIXED_M : !fft_fixed_length(pl.L); }
 
 void launch_fft_rows_fwd_real(const float* img, int W, int H, const FftPlan& plw, int ph, float2* out, cudaStream_t st) {
-  int T = runtime_plan(plw) ? rt_threads(plw, 1) : fft_threads(fft_work_len(plw), 1);
   size_t sm = 2 * fbytes(fft_work_len(plw), 1);
+  int T = runtime_plan(plw) ? rt_threads(plw, 1, sm) : fft_threads(fft_work_len(plw), 1);
   by_plan(plw, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
     set_smem((const void*)k_fft_rows_fwd_real<FL>, sm);
@@ -1437,8 +1507,8 @@ void launch_fft_rows_fwd_real(const float* img, int W, int H, const FftPlan& plw
 static void cols_fwd(float2* T, const FftPlan& plh, int pw, cudaStream_t st) {
   constexpr int C = 2;
   const int wh = fft_work_len(plh);
-  int nt = runtime_plan(plh) ? rt_threads(plh, C) : std::min(fft_threads(wh, C), COLS_TMAX);
   size_t sm_f = 2 * (size_t)fft_buf_stride(wh, C) * sizeof(float2);
+  int nt = runtime_plan(plh) ? rt_threads(plh, C, sm_f) : std::min(fft_threads(wh, C), COLS_TMAX);
   // in place: a block reads its C columns whole before it writes their spectrum back
   by_plan(plh, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
@@ -1454,17 +1524,37 @@ static void cols_inverse(const float2* S, const FftPlan& plh, int pw, const Gabo
                          cudaStream_t st) {
   constexpr int C = 2;
   const int ph = plh.L, wh = fft_work_len(plh);
-  int nt = runtime_plan(plh) ? rt_threads(plh, C) : std::min(fft_threads(wh, C), COLS_TMAX);
-  const size_t sm_p = smem_cols_pair(ph, wh);
+  const bool rt = runtime_plan(plh);
+  const size_t sm_p = smem_cols(ph, wh, 2);
+  auto launch_cols = [&](auto fl, auto cc, int nt, size_t sm) {
+    constexpr int FL = decltype(fl)::value, CC = decltype(cc)::value;
+    const void* fn = (const void*)k_fft_cols_pair<REFPACK, FL, CC>;
+    set_smem(fn, sm);
+    const int cols = (int)div_up(pw, CC);
+    if constexpr (REFPACK) {
+      OFC_LAUNCH((k_fft_cols_pair<true, FL, CC>), dim3(cols, 3), nt, sm, st, S, plh, pw, g, k0, k1, U);
+    } else {
+      const int G = resp_group(cols, g.F, resident_blocks(fn, nt, sm));
+      OFC_LAUNCH((k_fft_cols_pair<false, FL, CC>), dim3(cols, div_up(g.F, G)), nt, sm, st, S, plh, pw, g, 0, G, U);
+    }
+  };
+  // One column per block where the pair's buffers leave room for too few blocks (Bluestein's lengths of large radices
+  // above about 2700; the estimate of rt_threads, a column's 8-byte accesses counted 10 %): 911 x 1367 (M = 2873)
+  // 0.641 -> 0.510 ms per launch of the responses. Not at M = 4096 (1900 x 1977: 1.73 against 1.94 ms).
+  int nt = std::min(fft_threads(wh, C), COLS_TMAX);
+  if (rt) {
+    double t1 = 1e300, t2 = 1e300;
+    const size_t sm1 = smem_cols(ph, wh, 1);
+    const int n1 = rt_threads(plh, 1, sm1, &t1);
+    nt = rt_threads(plh, C, std::min(sm_p, SMEM_MAX), &t2);
+    if (plh.M && sm_p <= SMEM_MAX && 1.1 * t1 < 0.5 * t2) {
+      launch_cols(std::integral_constant<int, -1>{}, std::integral_constant<int, 1>{}, n1, sm1);
+      return;
+    }
+  }
   if (sm_p <= SMEM_MAX) {
     if (fft_fixed_length(ph)) nt = pair_threads<REFPACK>(ph);  // the block size the fixed-length kernel assumes
-    dim3 grid(div_up(pw, C), REFPACK ? 3 : div_up(g.F, RESP_G));
-    by_plan(plh, [&](auto fl) {
-      constexpr int FL = decltype(fl)::value;
-      set_smem((const void*)k_fft_cols_pair<REFPACK, FL>, sm_p);
-      if constexpr (REFPACK) OFC_LAUNCH((k_fft_cols_pair<true, FL>), grid, nt, sm_p, st, S, plh, pw, g, k0, k1, U);
-      else OFC_LAUNCH((k_fft_cols_pair<false, FL>), grid, nt, sm_p, st, S, plh, pw, g, k0, k1, U);
-    });
+    by_plan(plh, [&](auto fl) { launch_cols(fl, std::integral_constant<int, 2>{}, nt, sm_p); });
     return;
   }
   size_t sm_i = REFPACK ? 2 * fbytes(wh, C) : smem_prefilter(wh, C, nt);
@@ -1488,8 +1578,8 @@ void launch_fft_rows_inv_resp(const float2* U, const FftPlan& plw, int ph, int F
   const float scale = (float)(36.0 / ((double)ph * (double)plw.L));
   const int nrows = ((F + 1) / 2) * ph;
   if (runtime_plan(plw)) {
-    const int T = rt_threads(plw, 1);
     const size_t sm = (2 * (size_t)fft_buf_stride(plw.L, 1) + 2 * (size_t)fft_buf_stride(fft_work_len(plw), 1)) * sizeof(float2);
+    const int T = rt_threads(plw, 1, sm);
     auto launch = [&](auto fl) {
       constexpr int FL = decltype(fl)::value;
       set_smem((const void*)k_fft_rows_inv_resp_rt<FL>, sm);
@@ -1523,11 +1613,11 @@ void launch_fft_rows_inv_ref_f32(const float2* U, const FftPlan& plw, int ph, in
                                  float4* ref4, float* amp, cudaStream_t st) {
   const bool rt = runtime_plan(plw);
   const size_t wl = fft_buf_stride(fft_work_len(plw), 1);
-  int T = rt ? rt_threads(plw, 1) : fft_threads(fft_work_len(plw), 1);
   size_t sm = 4 * wl * sizeof(float2);
   const size_t sm2 = (3 * (size_t)fft_buf_stride(plw.L, 1) + 2 * wl) * sizeof(float2);
   const bool two = rt && sm2 <= SMEM_MAX;
   if (two) sm = sm2;
+  int T = rt ? rt_threads(plw, 1, sm) : fft_threads(fft_work_len(plw), 1);
   dim3 grid(H, k1 - k0);
   by_plan(plw, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
@@ -1537,8 +1627,8 @@ void launch_fft_rows_inv_ref_f32(const float2* U, const FftPlan& plw, int ph, in
 }
 
 void launch_fft_lines(float2* data, int lines, const FftPlan& pl, bool inverse, cudaStream_t st) {
-  int T = runtime_plan(pl) ? rt_threads(pl, 1) : fft_threads(fft_work_len(pl), 1);
   size_t sm = 2 * fbytes(fft_work_len(pl), 1);
+  int T = runtime_plan(pl) ? rt_threads(pl, 1, sm) : fft_threads(fft_work_len(pl), 1);
   by_plan(pl, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
     set_smem((const void*)k_fft_lines<FL>, sm);

@@ -17,7 +17,7 @@ bool fft_fixed_length(int L);
 constexpr int FFT_FIXED_M = 1216;
 constexpr int FFT_E = 8;       // complex values per thread (sets the threads of a block)
 constexpr int FFT_TMAX = 512;  // threads per block at most
-constexpr int RT_T = 256;      // the same of the runtime plans' kernels
+constexpr int RT_T = 768;      // the same of the runtime plans' kernels (80 registers)
 
 // A 1-D plan of length L: mixed-radix Stockham stages (radix p[i], stride s[i] = product of the radices
 // before it) and the twiddle table W[t] = exp(-2 pi i t / L), t < L, rounded from float64. Stage i's twiddles lie together
