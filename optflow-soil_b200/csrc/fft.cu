@@ -193,6 +193,7 @@ FftPlan fft_make_plan(int L, int variant) {
   std::vector<int> f = factor_order(work, fft_fixed_length(work) || work == FFT_FIXED_M ? 0 : variant);
   if (f.empty() || (int)f.size() > FFT_MAXST)
     throw Error(OFC_ERR_WINDOW, "FFT length " + std::to_string(L) + " needs too many stages");
+  pl.inner = pl.M && f == factor_order(work, 0) ? work : 0;
   int s = 1;
   pl.nst = (int)f.size();
   for (int i = 0; i < pl.nst; i++) {
@@ -726,21 +727,26 @@ constexpr CPlan cplan(int L) {
   return c;
 }
 
+// whether stage st of a fixed plan writes the padded layout (as fft_stage decides for the runtime plans)
+constexpr bool stage_pads(const CPlan& P, int st, int C) { return P.p[st] % 2 == 0 && st + 1 < P.nst && P.s[st] * C < 32; }
+
 // the fixed plan of length L from stage ST on: stage 0 reads `first` through IN, the last stage writes through OUT; the
-// stages write b, a, b, ... (ST = 0: first may be a); returns the buffer holding the result
+// stages write b, a, b, ... (ST = 0: first may be a), the last one dst where that is not null (neither buffer); returns
+// the buffer holding the result
 template <int L, int C, int ST, int IN, int OUT>
-__device__ __forceinline__ float2* fft_run_fixed(const float2* first, float2* a, float2* b, const FftPlan& pl, bool inv,
-                                                 const StageEx& ex) {
+__device__ __forceinline__ float2* fft_run_fixed(const float2* first, float2* a, float2* b, float2* dst, const FftPlan& pl,
+                                                 bool inv, const StageEx& ex) {
   constexpr CPlan P = cplan(L);
   if constexpr (ST == P.nst) {
     return a;
   } else {
-    constexpr int OSH = (ST + 1 < P.nst && P.s[ST] * C < 32) ? FFT_PAD : 31;
-    constexpr int ISH = ST == 0 ? 31 : (P.s[ST - 1] * C < 32 ? FFT_PAD : 31);
+    constexpr int OSH = stage_pads(P, ST, C) ? FFT_PAD : 31;
+    constexpr int ISH = ST > 0 && stage_pads(P, ST > 0 ? ST - 1 : 0, C) ? FFT_PAD : 31;
+    float2* to = ST + 1 == P.nst && dst ? dst : b;
     stage_fixed<P.p[ST], P.s[ST], L, C, ISH, OSH, ST == 0 ? IN : (int)IN_PLAIN, ST + 1 == P.nst ? OUT : (int)OUT_PLAIN>(
-        smem_addr(first), smem_addr(b), pl.stw + P.so[ST] + (inv ? P.nstw : 0), inv, ex);
+        smem_addr(first), smem_addr(to), pl.stw + P.so[ST] + (inv ? P.nstw : 0), inv, ex);
     __syncthreads();
-    return fft_run_fixed<L, C, ST + 1, IN, OUT>(b, b, a, pl, inv, ex);
+    return fft_run_fixed<L, C, ST + 1, IN, OUT>(b, to, a, dst, pl, inv, ex);
   }
 }
 
@@ -809,20 +815,49 @@ __device__ __forceinline__ float2* fft_stages(const float2* first, float2* a, fl
   return dst;
 }
 
+// The 16 inner lengths that fft_work_length gives most of the 1316 lengths from 160 to 2048 with a prime factor above 31
+// (the 16th serves 26 of them, all together 69 %; a further length costs 13 s of compile time and serves under 2 %).
+#define FFT_INNER_LENGTHS(X) \
+  X(1352) X(1463) X(1573) X(1672) X(1859) X(1976) X(2197) X(2431)                                  \
+  X(2527) X(2717) X(2873) X(3211) X(3328) X(3584) X(3757) X(4096)
+
+// Bluestein with the inner length FM fixed at compile time (L still read at run time): fft_bluestein's contract
+template <int FM, int LC, int IN>
+__device__ __noinline__ float2* fft_bluestein_fixed(const float2* first, float2* a, float2* b, float2* dst,
+                                                    const FftPlan& pl, bool inv, StageEx ex) {
+  constexpr int C = 1 << LC, CHIRP = IN == IN_MUL ? (int)IN_MULCHIRP : (int)IN_CHIRP;
+  float2* r = fft_run_fixed<FM, C, 0, CHIRP, OUT_FILT>(first, a, b, nullptr, pl, false, ex);
+  return fft_run_fixed<FM, C, 0, IN_PLAIN, OUT_CHIRP>(r, r, r == a ? b : a, dst, pl, true, ex);
+}
+
 // Bluestein (the plan's M > 0): X_k = w_k sum_n (x_n w_n) conj(w_{k - n}), w_n = exp(-i pi n^2 / L), the convolution
 // cyclic over M >= 2L - 1 by two length-M transforms; the inverse transform as conj(forward(conj(x))). The products by
 // the chirp and the filter are made as the transforms' first stages load and their last stages store. `first` holds the
 // line's L values (x C); a and b fft_buf_len(M, C) values each (first may be a); the result goes to dst (its L values;
-// may be `first`), or for a null dst to a or b.
-template <int LC, int IN>
+// may be `first`), or for a null dst to a or b. FM > 0: M is FM. The inner lengths that the most padded sizes take
+// (FFT_INNER_LENGTHS) have stages of their own, compiled for the default factor order: the strides, offsets and the
+// quotient by them are constants, where the runtime stages, bound by issued instructions, spend a third of them there
+// (response row pass: M = 2873, 1367 x 911, 444 -> 352 us; 1859, 853 x 1475, 505 -> 346 us; 4096, 1900 x 1977,
+// 1267 -> 980 us; the same values). Other inner lengths, and a plan in another factor order, run the runtime stages.
+template <int LC, int IN, int FM = 0>
 __device__ __forceinline__ float2* fft_bluestein(const float2* first, float2* a, float2* b, float2* dst, const FftPlan& pl,
                                                  bool inv, StageEx ex) {
   ex.L = pl.L;
   ex.conj = inv;
   ex.w = pl.chirp;
   ex.f = pl.filt;
-  float2* r = fft_stages<LC, IN == IN_MUL ? IN_MULCHIRP : IN_CHIRP, OUT_FILT>(first, a, b, nullptr, pl, pl.M, false, ex);
-  return fft_stages<LC, IN_PLAIN, OUT_CHIRP>(r, r, r == a ? b : a, dst, pl, pl.M, true, ex);
+  if constexpr (FM > 0) {
+    return fft_bluestein_fixed<FM, LC, IN>(first, a, b, dst, pl, inv, ex);
+  } else {
+    switch (pl.inner) {
+#define INNER_CASE(M) case M: return fft_bluestein_fixed<M, LC, IN>(first, a, b, dst, pl, inv, ex);
+      FFT_INNER_LENGTHS(INNER_CASE)
+#undef INNER_CASE
+      default: break;
+    }
+    float2* r = fft_stages<LC, IN == IN_MUL ? IN_MULCHIRP : IN_CHIRP, OUT_FILT>(first, a, b, nullptr, pl, pl.M, false, ex);
+    return fft_stages<LC, IN_PLAIN, OUT_CHIRP>(r, r, r == a ? b : a, dst, pl, pl.M, true, ex);
+  }
 }
 
 // a runtime plan's transform of the line(s) in `first` (L values x C, not kept) with two scratch buffers of
@@ -831,18 +866,6 @@ template <int FIXL, int LC>
 __device__ __forceinline__ void fft_run_to(const float2* first, float2* a, float2* b, float2* dst, const FftPlan& pl, bool inv) {
   if constexpr (FIXL == -1) fft_bluestein<LC, IN_PLAIN>(first, a, b, dst, pl, inv, StageEx{});
   else fft_stages<LC, IN_PLAIN, OUT_PLAIN>(first, a, b, dst, pl, pl.L, inv, StageEx{});
-}
-
-// Bluestein with the inner length FM fixed at compile time (L still read at run time); the result in a or b
-template <int FM, int C, int IN>
-__device__ __forceinline__ float2* fft_bluestein_fixed(const float2* first, float2* a, float2* b, const FftPlan& pl, bool inv,
-                                                       StageEx ex) {
-  ex.L = pl.L;
-  ex.conj = inv;
-  ex.w = pl.chirp;
-  ex.f = pl.filt;
-  float2* r = fft_run_fixed<FM, C, 0, IN == IN_MUL ? (int)IN_MULCHIRP : (int)IN_CHIRP, OUT_FILT>(first, a, b, pl, false, ex);
-  return fft_run_fixed<FM, C, 0, IN_PLAIN, OUT_CHIRP>(r, r, r == a ? b : a, pl, true, ex);
 }
 
 // runs the plan on buf (tmp: scratch of the same capacity, fft_buf_len(fft_work_len(pl), C)); buf holds the input
@@ -855,11 +878,11 @@ __device__ C2* fft_run(C2* buf, C2* tmp, const FftPlan& pl, bool inv) {
   static_assert(std::is_same<C2, float2>::value, "float32 transforms");
   constexpr int LC = C == 2 ? 1 : 0;
   if constexpr (FIXL > 0) {
-    return fft_run_fixed<FIXL, C, 0, IN_PLAIN, OUT_PLAIN>(buf, buf, tmp, pl, inv, StageEx{});
+    return fft_run_fixed<FIXL, C, 0, IN_PLAIN, OUT_PLAIN>(buf, buf, tmp, nullptr, pl, inv, StageEx{});
   } else if constexpr (FIXL == -1) {  // the kernels' instantiation for Bluestein plans (pl.M > 0)
     return fft_bluestein<LC, IN_PLAIN>(buf, buf, tmp, nullptr, pl, inv, StageEx{});
   } else if constexpr (FIXL < -1) {  // Bluestein with the inner length -FIXL fixed at compile time
-    return fft_bluestein_fixed<-FIXL, C, IN_PLAIN>(buf, buf, tmp, pl, inv, StageEx{});
+    return fft_bluestein<LC, IN_PLAIN, -FIXL>(buf, buf, tmp, nullptr, pl, inv, StageEx{});
   } else {
     return fft_stages<LC, IN_PLAIN, OUT_PLAIN>(buf, buf, tmp, nullptr, pl, pl.L, inv, StageEx{});
   }
@@ -1042,13 +1065,20 @@ __global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? COLS_TMAX : RT_T, FIXL
 // Bluestein plans whose pair would leave an SM's shared memory room for too few blocks.
 
 // threads of the fixed-length column-pair kernel: the responses COLS_TMAX; the reference pack, whose float64 factors
-// take more time per element, one per radix-8 butterfly of the two columns (2 x 2112 / 8)
-constexpr int PAIR_T_REF = 544;
+// take more time per element, one per radix-8 butterfly of the two columns (2 x 2112 / 8); the fixed inner length
+// (1216 = 8 8 19: 304 radix-8 butterflies, 128 of radix 19) 256 in 3 blocks per SM (960 x 540: 179 -> 173 us against
+// COLS_TMAX in 2, the reference pack 232 -> 225 us)
+constexpr int PAIR_T_REF = 544, PAIR_T_INNER = 256;
 template <bool REFPACK>
-constexpr int pair_threads(int fixl) { return fixl > 0 && REFPACK ? PAIR_T_REF : (fixl == 0 || fixl == -1 ? RT_T : COLS_TMAX); }
+constexpr int pair_threads(int fixl) {
+  if (fixl > 0) return REFPACK ? PAIR_T_REF : COLS_TMAX;
+  return fixl < -1 ? PAIR_T_INNER : RT_T;
+}
+constexpr int pair_minb(int fixl) { return fixl > 0 ? 2 : (fixl < -1 ? 3 : RT_MINB); }
 template <bool REFPACK, int FIXL, int C>
-__global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), FIXL == 0 || FIXL == -1 ? RT_MINB : 2) k_fft_cols_pair(const float2* __restrict__ S, FftPlan plh, int pw,
-                                                                GaborTables g, int k0, int k1, float2* __restrict__ U) {
+__global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), pair_minb(FIXL))
+    k_fft_cols_pair(const float2* __restrict__ S, FftPlan plh, int pw, GaborTables g, int k0, int k1,
+                    float2* __restrict__ U) {
   static_assert(C == 2 || FIXL == -1, "one column per block: Bluestein's runtime plans");
   constexpr int LC = C - 1;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1107,8 +1137,8 @@ __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), FIXL == 0 || FIXL
       ex.omx = omx;
       ex.exb = exb;
       float2* r;
-      if constexpr (FIXL > 0) r = fft_run_fixed<FIXL, C, 0, IN_MUL, OUT_PLAIN>(raw, A, B, plh, true, ex);
-      else if constexpr (FIXL < -1) r = fft_bluestein_fixed<-FIXL, C, IN_MUL>(raw, A, B, plh, true, ex);
+      if constexpr (FIXL > 0) r = fft_run_fixed<FIXL, C, 0, IN_MUL, OUT_PLAIN>(raw, A, B, nullptr, plh, true, ex);
+      else if constexpr (FIXL < -1) r = fft_bluestein<LC, IN_MUL, -FIXL>(raw, A, B, nullptr, plh, true, ex);
       else if constexpr (FIXL == 0) r = fft_stages<LC, IN_MUL, OUT_PLAIN>(raw, A, B, nullptr, plh, ph, true, ex);
       else r = fft_bluestein<LC, IN_MUL>(raw, A, B, nullptr, plh, true, ex);
       float2* idle = r == A ? B : A;
@@ -1554,6 +1584,7 @@ static void cols_inverse(const float2* S, const FftPlan& plh, int pw, const Gabo
   }
   if (sm_p <= SMEM_MAX) {
     if (fft_fixed_length(ph)) nt = pair_threads<REFPACK>(ph);  // the block size the fixed-length kernel assumes
+    else if (plh.M == FFT_FIXED_M) nt = std::min(nt, pair_threads<REFPACK>(-FFT_FIXED_M));
     by_plan(plh, [&](auto fl) { launch_cols(fl, std::integral_constant<int, 2>{}, nt, sm_p); });
     return;
   }

@@ -23,7 +23,8 @@ constexpr int RT_T = 768;      // the same of the runtime plans' kernels (80 reg
 // before it) and the twiddle table W[t] = exp(-2 pi i t / L), t < L, rounded from float64. Stage i's twiddles lie together
 // as its butterflies read them, stw[so[i] + (k - 1) m + q] = W[k q s[i]] (m = L / (p[i] s[i]), k = 1 .. p[i] - 1, q < m):
 // neighbouring threads (consecutive q) read neighbouring values, where W itself is read at a stride of k s[i]; the nstw
-// values are followed by their conjugates (the inverse transform's).
+// values are followed by their conjugates (the inverse transform's). inner: M where its stages are in the default order
+// (the transforms of the common inner lengths are compiled for that order), else 0.
 // A length with a prime factor above 31 is transformed by Bluestein's chirp z-transform (as the reference's Metal
 // FFT does, rust/crates/optflow-gpu/src/fft.rs:1-3): M > 0 is then the inner length (a length >= 2L - 1 of
 // the radices with butterflies, of fewest stages: fft_work_length), the stages and tw are those of length M, chirp[n] = exp(-i pi n^2 / L) for n < L, and filt is the
@@ -38,6 +39,7 @@ struct FftPlan {
   const float2* tw = nullptr;
   const float2* stw = nullptr;
   int nstw = 0;
+  int inner = 0;
   int M = 0;
   const float2* chirp = nullptr;
   const float2* filt = nullptr;

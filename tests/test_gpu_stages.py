@@ -39,6 +39,31 @@ def test_fft_lines_runtime_plans(T, L, bound):
         assert np.abs(got - ref).max() < bound * np.abs(ref).max(), (L, inv)
 
 
+@pytest.mark.parametrize("variant", [0, 3])
+@pytest.mark.parametrize("L", [674, 705, 787, 811, 929, 958, 1099, 1214, 1241, 1328, 1437, 1606, 1637, 1791, 1821, 2047])
+def test_fft_lines_compiled_inner_lengths(T, L, variant):
+    """One length of each Bluestein inner length with stages of its own (1352 ... 4096), in the default factor order and
+    reversed (which those stages do not serve); the Bluestein bound of test_fft_lines_match_numpy."""
+    from optflow_b200 import Engine, _abi
+    lib = _abi.load()
+
+    def order(v):
+        n, var = np.array([L], np.int32), np.array([v], np.int32)
+        lib.ofc_fft_set_plans(n.ctypes.data_as(_abi.c_i32_p), var.ctypes.data_as(_abi.c_i32_p), 1)
+
+    rng = np.random.default_rng(L)
+    a = (rng.standard_normal((3, L)) + 1j * rng.standard_normal((3, L))).astype(np.complex64)
+    fwd = np.fft.fft(a.astype(np.complex128), axis=1)
+    inv = np.fft.ifft(a.astype(np.complex128), axis=1) * L
+    order(variant)
+    try:
+        eng = Engine(0)  # a fresh engine builds its plan from the table
+        for inverse, ref in ((False, fwd), (True, inv)):
+            assert np.abs(T.fft_lines(a, inverse=inverse, engine=eng) - ref).max() < 1e-5 * np.abs(ref).max(), inverse
+    finally:
+        order(0)
+
+
 @pytest.mark.parametrize("shape", [(133, 911), (40, 1367), (1367, 75), (185, 333), (40, 5936), (777, 68), (40, 777), (1977, 70)])
 def test_passes_runtime_plans(T, oracle, shape):
     """The row and column passes on runtime plans (direct, Bluestein, odd pitches; 6000 padded columns, where the
