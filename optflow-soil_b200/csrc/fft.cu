@@ -1003,6 +1003,7 @@ __host__ __device__ constexpr int fft_buf_stride(int L, int C) { return (fft_buf
 template <int FIXL>
 __global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? FFT_TMAX : RT_T, FIXL > 0 || FIXL < -1 ? 2 : RT_MINB) k_fft_rows_fwd_real(const float* __restrict__ img, int W, int H,
                                                                   FftPlan plw, int ph, float2* __restrict__ out) {
+  grid_dep_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* sm = (float2*)smraw;
   const int pw = FIXL > 0 ? FIXL : plw.L;
@@ -1025,6 +1026,7 @@ constexpr int COLS_TMAX = 320;  // threads per block of the split column pass
 
 template <int C, int FIXL>
 __global__ void __launch_bounds__(FIXL > 0 || FIXL < -1 ? COLS_TMAX : RT_T, FIXL > 0 || FIXL < -1 ? 3 : RT_MINB) k_fft_cols_fwd(const float2* Tin, FftPlan plh, int pw, float2* S) {
+  grid_dep_wait();
   constexpr int LC = C == 4 ? 2 : (C == 2 ? 1 : 0);
   extern __shared__ __align__(16) unsigned char smraw[];
   float2* A = (float2*)smraw;
@@ -1079,6 +1081,7 @@ template <bool REFPACK, int FIXL, int C>
 __global__ void __launch_bounds__(pair_threads<REFPACK>(FIXL), pair_minb(FIXL))
     k_fft_cols_pair(const float2* __restrict__ S, FftPlan plh, int pw, GaborTables g, int k0, int k1,
                     float2* __restrict__ U) {
+  grid_dep_wait();
   static_assert(C == 2 || FIXL == -1, "one column per block: Bluestein's runtime plans");
   constexpr int LC = C - 1;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1258,6 +1261,7 @@ template <int FIXL>
 __global__ void __launch_bounds__(FIXL > 0 ? 288 : FFT_TMAX, FIXL > 0 ? 3 : 2)
     k_fft_rows_inv_resp(const float2* __restrict__ U, FftPlan plw, int ph, int F, int nrows, float scale,
                         float2* __restrict__ R) {
+  grid_dep_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int L = FIXL > 0 ? FIXL : plw.L, nb = fft_buf_stride(FIXL > 0 ? FIXL : fft_work_len(plw), 1);
   float2* b0 = (float2*)smraw;
@@ -1318,6 +1322,7 @@ __global__ void __launch_bounds__(FIXL > 0 ? 288 : FFT_TMAX, FIXL > 0 ? 3 : 2)
 template <int FIXL>
 __global__ void __launch_bounds__(RT_T, RT_MINB) k_fft_rows_inv_resp_rt(const float2* __restrict__ U, FftPlan plw, int ph, int F,
                                                                   float scale, float2* __restrict__ R) {
+  grid_dep_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int L = plw.L, nl = fft_buf_stride(L, 1), nb = fft_buf_stride(fft_work_len(plw), 1), row = blockIdx.x;
   float2 *x0 = (float2*)smraw, *x1 = x0 + nl, *a = x1 + nl, *b = a + nb;
@@ -1530,7 +1535,7 @@ void launch_fft_rows_fwd_real(const float* img, int W, int H, const FftPlan& plw
   by_plan(plw, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
     set_smem((const void*)k_fft_rows_fwd_real<FL>, sm);
-    OFC_LAUNCH(k_fft_rows_fwd_real<FL>, ph, T, sm, st, img, W, H, plw, ph, out);
+    OFC_LAUNCH_PDL(k_fft_rows_fwd_real<FL>, ph, T, sm, st, img, W, H, plw, ph, out);
   });
 }
 
@@ -1543,7 +1548,7 @@ static void cols_fwd(float2* T, const FftPlan& plh, int pw, cudaStream_t st) {
   by_plan(plh, [&](auto fl) {
     constexpr int FL = decltype(fl)::value;
     set_smem((const void*)k_fft_cols_fwd<C, FL>, sm_f);
-    OFC_LAUNCH((k_fft_cols_fwd<C, FL>), div_up(pw, C), nt, sm_f, st, T, plh, pw, T);
+    OFC_LAUNCH_PDL((k_fft_cols_fwd<C, FL>), div_up(pw, C), nt, sm_f, st, T, plh, pw, T);
   });
 }
 
@@ -1562,10 +1567,10 @@ static void cols_inverse(const float2* S, const FftPlan& plh, int pw, const Gabo
     set_smem(fn, sm);
     const int cols = (int)div_up(pw, CC);
     if constexpr (REFPACK) {
-      OFC_LAUNCH((k_fft_cols_pair<true, FL, CC>), dim3(cols, 3), nt, sm, st, S, plh, pw, g, k0, k1, U);
+      OFC_LAUNCH_PDL((k_fft_cols_pair<true, FL, CC>), dim3(cols, 3), nt, sm, st, S, plh, pw, g, k0, k1, U);
     } else {
       const int G = resp_group(cols, g.F, resident_blocks(fn, nt, sm));
-      OFC_LAUNCH((k_fft_cols_pair<false, FL, CC>), dim3(cols, div_up(g.F, G)), nt, sm, st, S, plh, pw, g, 0, G, U);
+      OFC_LAUNCH_PDL((k_fft_cols_pair<false, FL, CC>), dim3(cols, div_up(g.F, G)), nt, sm, st, S, plh, pw, g, 0, G, U);
     }
   };
   // One column per block where the pair's buffers leave room for too few blocks (Bluestein's lengths of large radices
@@ -1614,7 +1619,7 @@ void launch_fft_rows_inv_resp(const float2* U, const FftPlan& plw, int ph, int F
     auto launch = [&](auto fl) {
       constexpr int FL = decltype(fl)::value;
       set_smem((const void*)k_fft_rows_inv_resp_rt<FL>, sm);
-      OFC_LAUNCH(k_fft_rows_inv_resp_rt<FL>, nrows, T, sm, st, U, plw, ph, F, scale, R);
+      OFC_LAUNCH_PDL(k_fft_rows_inv_resp_rt<FL>, nrows, T, sm, st, U, plw, ph, F, scale, R);
     };
     if (plw.M) launch(std::integral_constant<int, -1>{});
     else launch(std::integral_constant<int, 0>{});
@@ -1627,7 +1632,7 @@ void launch_fft_rows_inv_resp(const float2* U, const FftPlan& plw, int ph, int F
     if constexpr (FL > 0 || FL < -1) {
       const void* fn = (const void*)k_fft_rows_inv_resp<FL>;
       set_smem(fn, sm);
-      OFC_LAUNCH(k_fft_rows_inv_resp<FL>, persistent_blocks(fn, T, sm, nrows), T, sm, st, U, plw, ph, F, nrows, scale,
+      OFC_LAUNCH_PDL(k_fft_rows_inv_resp<FL>, persistent_blocks(fn, T, sm, nrows), T, sm, st, U, plw, ph, F, nrows, scale,
                  R);
     }
   });

@@ -52,6 +52,7 @@ constexpr int CORR_R = 16, CY_RY = 8, CX_RX = 3;
 
 __global__ void __launch_bounds__(128, 6) k_corr_y_rb(const double* __restrict__ in, double* __restrict__ out, int W,
                                                      int H, const double* __restrict__ taps) {
+  grid_dep_wait();
   constexpr int R = CORR_R, RY = CY_RY, NV = RY + 2 * R;
   __shared__ double tk[R + 1];
   if (threadIdx.x <= R) tk[threadIdx.x] = taps[R + threadIdx.x];
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(128, 6) k_corr_y_rb(const double* __restrict__
 
 __global__ void __launch_bounds__(128) k_corr_x_rb(const double* __restrict__ in, double* __restrict__ out, int W, int H,
                                                   const double* __restrict__ taps) {
+  grid_dep_wait();
   constexpr int R = CORR_R, RX = CX_RX, NT = 128, SEG = NT * RX, WIN = SEG + 2 * R, NV = RX + 2 * R;
   __shared__ double tk[R + 1];
   __shared__ double wb[WIN];
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(128) k_corr_x_rb(const double* __restrict__ in
 void launch_corr_y(const double* in, double* out, int n_planes, int W, int H, const double* taps, int r, cudaStream_t st) {
   if (r == CORR_R) {
     dim3 g(div_up(W, 128), div_up(H, CY_RY), n_planes);
-    OFC_LAUNCH(k_corr_y_rb, g, 128, 0, st, in, out, W, H, taps);
+    OFC_LAUNCH_PDL(k_corr_y_rb, g, 128, 0, st, in, out, W, H, taps);
     return;
   }
   dim3 g(div_up(W, 128), H, n_planes);
@@ -120,7 +122,7 @@ void launch_corr_y(const double* in, double* out, int n_planes, int W, int H, co
 void launch_corr_x(const double* in, double* out, int n_planes, int W, int H, const double* taps, int r, cudaStream_t st) {
   if (r == CORR_R) {
     dim3 g(div_up(W, 128 * CX_RX), H, n_planes);
-    OFC_LAUNCH(k_corr_x_rb, g, 128, 0, st, in, out, W, H, taps);
+    OFC_LAUNCH_PDL(k_corr_x_rb, g, 128, 0, st, in, out, W, H, taps);
     return;
   }
   dim3 g(div_up(W, 128), H, n_planes);
@@ -323,6 +325,7 @@ void launch_bspline_f32(const float* in, float* out, double* tmp, int W, int H, 
 // ---------------------------------------------------------------- warp
 __global__ void __launch_bounds__(128, 8) k_warp(const float* __restrict__ c2, int w2, int h2, const double* __restrict__ sx,
                        const double* __restrict__ sy, long shx, long shy, int W, int H, float* __restrict__ out) {
+  grid_dep_wait();
   int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= W) return;
   for (int y = blockIdx.y; y < H; y += gridDim.y) {  // rows beyond the grid's 65535 in steps of gridDim.y
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(128, 8) k_warp(const float* __restrict__ c2, i
 void launch_warp_gather(const float* c2, int w2, int h2, const double* sx, const double* sy, long shx, long shy, int W,
                         int H, float* out, cudaStream_t st) {
   dim3 g(div_up(W, 128), (unsigned)std::min(H, 65535));
-  OFC_LAUNCH(k_warp, g, 128, 0, st, c2, w2, h2, sx, sy, shx, shy, W, H, out);
+  OFC_LAUNCH_PDL(k_warp, g, 128, 0, st, c2, w2, h2, sx, sy, shx, shy, W, H, out);
 }
 
 // ---------------------------------------------------------------- accumulate
@@ -456,6 +459,7 @@ __global__ void __launch_bounds__(ACC_T, ACC_MINB) k_accumulate(const float4* __
                                                       const double* __restrict__ uy, const double* __restrict__ sx,
                                                       const double* __restrict__ sy, const double2* __restrict__ cs,
                                                       int W, int H, double* __restrict__ sums) {
+  grid_dep_wait();
   extern __shared__ float4 pk[];  // ACC_ST x 2 x ACC_T
   // a block covers ACC_BX x ACC_BY pixels: its warps' response taps share rows in L1
   const int x = blockIdx.x * ACC_BX + threadIdx.x, y = blockIdx.y * ACC_BY + threadIdx.y;
@@ -573,7 +577,7 @@ void launch_accumulate_gather(const float4* ref4, const float2* R, int F, int ph
   if (F > ACC_MAXF)
     throw Error(OFC_ERR_WINDOW, "too many Gabor filters (" + std::to_string(F) + ") for the CUDA engine");
   raise_smem_limit((const void*)k_accumulate, sm);
-  OFC_LAUNCH(k_accumulate, g, dim3(ACC_BX, ACC_BY), sm, st, ref4, (const float4*)R, F, ph, pw, ux, uy, sx, sy, cs, W, H, sums);
+  OFC_LAUNCH_PDL(k_accumulate, g, dim3(ACC_BX, ACC_BY), sm, st, ref4, (const float4*)R, F, ph, pw, ux, uy, sx, sy, cs, W, H, sums);
 }
 
 // ---------------------------------------------------------------- window moments + solve
@@ -854,6 +858,7 @@ struct MomY {
 template <int ORDER>
 __global__ void __launch_bounds__(32 * MY_W, MomY<ORDER>::MINB) k_moments_y_rb(const double* __restrict__ sums, int W, int H, MomTaps tp,
                                                              double* __restrict__ yplanes) {
+  grid_dep_wait();
   constexpr int R = MOM_R, RY = MomY<ORDER>::RY, TB = MY_W * RY, NR = TB + 2 * R;
   static_assert(NR % MY_W == 0, "whole rows of the tile per warp");
   __shared__ double tile[NR * 32];
@@ -983,6 +988,7 @@ __global__ void __launch_bounds__(MomX<ORDER>::NT, MomX<ORDER>::MINB) k_moments_
                                                                MomTaps tp, double* __restrict__ oux,
                                                                double* __restrict__ ouy, double* __restrict__ energy,
                                                                double* __restrict__ resid, double* __restrict__ slope) {
+  grid_dep_wait();
   constexpr MomTable T = build_table(ORDER);
   constexpr int n = ORDER == 1 ? 6 : 12;
   constexpr int RX = MomX<ORDER>::RX, G = MomX<ORDER>::G, NT = MomX<ORDER>::NT, SEG = MomX<ORDER>::SEG;
@@ -1090,11 +1096,11 @@ static void launch_moments_rb(const double* sums, const double* ux, const double
                               double* yplanes, double* oux, double* ouy, double* energy, double* resid, double* slope,
                               cudaStream_t st) {
   dim3 gy(div_up(W, 32), div_up(H, MY_W * MomY<ORDER>::RY), 7);
-  OFC_LAUNCH(k_moments_y_rb<ORDER>, gy, 32 * MY_W, 0, st, sums, W, H, tp, yplanes);
+  OFC_LAUNCH_PDL(k_moments_y_rb<ORDER>, gy, 32 * MY_W, 0, st, sums, W, H, tp, yplanes);
   const size_t sm = MomX<ORDER>::smem();
   raise_smem_limit((const void*)k_moments_x_solve_rb<ORDER>, sm);
   dim3 gx(div_up(W, MomX<ORDER>::SEG), H);
-  OFC_LAUNCH(k_moments_x_solve_rb<ORDER>, gx, MomX<ORDER>::NT, sm, st, yplanes, ux, uy, W, H, tp, oux, ouy, energy, resid,
+  OFC_LAUNCH_PDL(k_moments_x_solve_rb<ORDER>, gx, MomX<ORDER>::NT, sm, st, yplanes, ux, uy, W, H, tp, oux, ouy, energy, resid,
              slope);
 }
 
@@ -1529,6 +1535,7 @@ template <int CAPT>
 __global__ void __launch_bounds__(WT_T) k_within_tile(const uint8_t* __restrict__ src, int W, int H, int cap_rt,
                                                       double limit, int mode, uint8_t* out, const int* gate,
                                                       int* count) {
+  grid_dep_wait();
   if (gate && *gate == 0) return;
   const int cap = CAPT ? CAPT : cap_rt;
   __shared__ uint8_t s[(WT_Y + 2 * WT_CAPMAX) * (WT_X + 2 * WT_CAPMAX)];
@@ -1610,9 +1617,9 @@ static void within(const uint8_t* src, int W, int H, double limit, int mode, uin
   if (cap <= WT_CAPMAX) {
     dim3 g(div_up(W, WT_X), div_up(H, WT_Y));
     if (cap == 13)  // the default radii (12.22 px)
-      OFC_LAUNCH(k_within_tile<13>, g, WT_T, 0, st, src, W, H, cap, limit, mode, out, gate, count);
+      OFC_LAUNCH_PDL(k_within_tile<13>, g, WT_T, 0, st, src, W, H, cap, limit, mode, out, gate, count);
     else
-      OFC_LAUNCH(k_within_tile<0>, g, WT_T, 0, st, src, W, H, cap, limit, mode, out, gate, count);
+      OFC_LAUNCH_PDL(k_within_tile<0>, g, WT_T, 0, st, src, W, H, cap, limit, mode, out, gate, count);
     return;
   }
   dim3 g(div_up(W, 128), H);
@@ -1632,6 +1639,7 @@ constexpr int CSEG = 64;
 
 __global__ void k_col_segments(const uint8_t* __restrict__ ok, int W, int H, const PrewarpCounts* c,
                                int* __restrict__ seg_first, int* __restrict__ seg_last) {
+  grid_dep_wait();
   if (!(c->low > 0 && c->ok > 0 && c->ok < W * H)) return;
   int x = blockIdx.x * blockDim.x + threadIdx.x;
   int sg = blockIdx.y;
@@ -1650,6 +1658,7 @@ __global__ void k_col_segments(const uint8_t* __restrict__ ok, int W, int H, con
 __global__ void k_col_nearest(const uint8_t* __restrict__ ok, int W, int H, const PrewarpCounts* c,
                               const int* __restrict__ seg_first, const int* __restrict__ seg_last,
                               int* __restrict__ col_d2, int* __restrict__ col_row) {
+  grid_dep_wait();
   if (!(c->low > 0 && c->ok > 0 && c->ok < W * H)) return;
   int x = blockIdx.x * blockDim.x + threadIdx.x;
   int y = blockIdx.y;
@@ -1686,6 +1695,7 @@ __global__ void k_extrapolate(const uint8_t* __restrict__ ok, const int* __restr
                               const int* __restrict__ col_row, const double* __restrict__ ux,
                               const double* __restrict__ uy, const double* __restrict__ slope, int W, int H,
                               const PrewarpCounts* c, double* ux_pre, double* uy_pre) {
+  grid_dep_wait();
   int x = blockIdx.x * blockDim.x + threadIdx.x;
   int y = blockIdx.y;
   if (x >= W) return;
@@ -1731,9 +1741,9 @@ void launch_prewarp_fill(const uint8_t* low, const double* ux, const double* uy,
   within(low, W, H, R, 1, ok, vdist, (const int*)&counts->low, &counts->ok, st);
   int* seg = vdist;  // the vertical distances are spent: 2 * ceil(H / CSEG) * W ints of segment summaries
   const int nseg = (H + CSEG - 1) / CSEG;
-  OFC_LAUNCH(k_col_segments, dim3(div_up(W, 128), nseg), 128, 0, st, ok, W, H, counts, seg, seg + (size_t)nseg * W);
-  OFC_LAUNCH(k_col_nearest, g, 128, 0, st, ok, W, H, counts, seg, seg + (size_t)nseg * W, col_d2, col_row);
-  OFC_LAUNCH(k_extrapolate, g, 128, 0, st, ok, col_d2, col_row, ux, uy, slope, W, H, counts, ux_pre, uy_pre);
+  OFC_LAUNCH_PDL(k_col_segments, dim3(div_up(W, 128), nseg), 128, 0, st, ok, W, H, counts, seg, seg + (size_t)nseg * W);
+  OFC_LAUNCH_PDL(k_col_nearest, g, 128, 0, st, ok, W, H, counts, seg, seg + (size_t)nseg * W, col_d2, col_row);
+  OFC_LAUNCH_PDL(k_extrapolate, g, 128, 0, st, ok, col_d2, col_row, ux, uy, slope, W, H, counts, ux_pre, uy_pre);
 }
 
 // ---------------------------------------------------------------- conversions
