@@ -38,6 +38,13 @@ OFC_API int ofc_test_local_solve(ofc_engine* eng, const double* sums, const doub
 /* np.median of n doubles. */
 OFC_API int ofc_test_median(ofc_engine* eng, const double* v, size_t n, double* median, char* err, size_t errlen);
 
+/* `rounds` energy medians and resets one after the other on one state, as a refinement runs them (phaseflow.py:149-161):
+ * round k takes the n energies at energy + k n, needs the median when force[k], and resets the pixels below the threshold
+ * to the field u (2 planes of n). medians[k]: the state's median after round k; planes + 7 k n: ux, uy, resid (zero before
+ * the round) and the 4 slope planes (NaN before). */
+OFC_API int ofc_test_median_reset(ofc_engine* eng, const double* energy, size_t rounds, size_t n, const uint8_t* force,
+                                  const double* u, double* medians, double* planes, char* err, size_t errlen);
+
 /* track._large_components (python/optflow_ref/track.py:45-53) of a w x h mask. */
 OFC_API int ofc_test_large_components(ofc_engine* eng, const uint8_t* b, size_t w, size_t h, double min_area,
                                       uint8_t* out, char* err, size_t errlen);

@@ -3238,6 +3238,34 @@ int ofc_test_median(ofc_engine* e, const double* v, size_t n, double* median, ch
   });
 }
 
+int ofc_test_median_reset(ofc_engine* e, const double* energy, size_t rounds, size_t n, const uint8_t* force,
+                          const double* u, double* medians, double* planes, char* err, size_t errlen) {
+  return guarded(e, err, errlen, [&](Lane& L) {
+    double* d = L.upload("t_med", energy, rounds * n);
+    double* du = L.upload("u2", u, 2 * n);
+    double* o = L.get<double>("u2b", 2 * n);
+    double* rs = L.get<double>("resid", n);
+    double* sl = L.get<double>("slope", 4 * n);
+    EnergyStats* stats = L.get<EnergyStats>("stats", 1);
+    unsigned long long* hist = L.get<unsigned long long>("hist", median_scratch(n));
+    launch_energy_stats_init(stats, hist, L.stream);
+    double* ek = L.get<double>("energy", n);
+    for (size_t k = 0; k < rounds; k++) {
+      OFC_CUDA(cudaMemcpyAsync(ek, d + k * n, n * 8, cudaMemcpyDeviceToDevice, L.stream));
+      OFC_CUDA(cudaMemsetAsync(o, 0, 2 * n * 8, L.stream));
+      OFC_CUDA(cudaMemsetAsync(rs, 0, n * 8, L.stream));
+      OFC_CUDA(cudaMemsetAsync(sl, 255, 4 * n * 8, L.stream));
+      launch_median_reset(ek, n, stats, (int)(k & 1), force[k] != 0, hist, du, du + n, o, o + n, rs, sl, L.stream);
+      double* out = planes + k * 7 * n;
+      OFC_CUDA(cudaMemcpyAsync(out, o, 2 * n * 8, cudaMemcpyDeviceToHost, L.stream));
+      OFC_CUDA(cudaMemcpyAsync(out + 2 * n, rs, n * 8, cudaMemcpyDeviceToHost, L.stream));
+      OFC_CUDA(cudaMemcpyAsync(out + 3 * n, sl, 4 * n * 8, cudaMemcpyDeviceToHost, L.stream));
+      OFC_CUDA(cudaMemcpyAsync(medians + k, &stats->median, 8, cudaMemcpyDeviceToHost, L.stream));
+      OFC_CUDA(cudaStreamSynchronize(L.stream));
+    }
+  });
+}
+
 int ofc_test_large_components(ofc_engine* e, const uint8_t* b, size_t w, size_t h, double min_area, uint8_t* out,
                               char* err, size_t errlen) {
   return guarded(e, err, errlen, [&](Lane& L) {

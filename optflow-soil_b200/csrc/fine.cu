@@ -1,11 +1,13 @@
 // fine.cu -- the per-pixel kernels of the fine stage (python/optflow_ref/phaseflow.py:427-511,
 // rust/crates/optflow-core/src/phaseflow.rs:1514-1613): smoothing, splines, warp, accumulate, window moments
 // and the local solve, the energy median, the confidence and the trusted pre-warp.
+#include <algorithm>
 #include <cfloat>
 #include <type_traits>
 
 #include "kernels.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_pipeline.h>
 
 namespace ofc {
@@ -1122,323 +1124,564 @@ void launch_moments_solve(const double* sums, const double* ux, const double* uy
   }
 }
 
-// ---------------------------------------------------------------- the energies' range
+// ---------------------------------------------------------------- energy median and reset
+// The median of the energy (np.median, phaseflow.py:149-151) by an exact select over order-preserving keys, and the reset
+// that reads it:
+// 1. the range of the energies and the reset rule (phaseflow.rs:846-854): when every energy is above 1e-9 max + 1e-30 no
+//    pixel is reset, and unless the caller needs the median nothing more is done;
+// 2. a histogram of 4096 equal parts of the keys' range, and the part that holds the element of rank n / 2;
+// 3. that part's elements as a candidate list, the largest key below it, and the select among the candidates (their range
+//    split again while there are more than MED_LIST, then by counting);
+// 4. the reset of each pixel below the threshold.
+// Blocks wait for each other only at the hardware's cluster barrier: no wait can give up, a median shares the SMs with
+// other streams' kernels, and the launches take programmatic dependencies like their neighbours. One cooperative launch of
+// 1024-thread blocks with grid barriers, as it was before, is no faster (us per pair before -> now: 128^2 1290 -> 1212, 256^2
+// 1637 -> 1612, 512^2 of order 2 4220 -> 4192, 1024^2 8690 -> 8610, 2048^2 30930 -> 30850).
+// Small images are bound by the launches' latency: up to MED_CLUSTER_N energies one cluster of 8 blocks does it all
+// (k_median_cluster; 300 x 300 pairs 2228 us against 2252 with a launch per step, 360 x 360 3623 against 3593). Beyond, a
+// launch per step over the whole chip, whose last block to finish picks (k_median_range, k_median_hist, k_median_select,
+// k_median_reset). With energies over 50 octaves (60 % of a frame dark) the candidates are many and one block's select of
+// them takes 10 us of a launch more (2048^2: 45.7 ms per pair, as before).
+constexpr size_t MED_CLUSTER_N = 98304;
 __device__ __forceinline__ unsigned long long okey(double v) {  // order-preserving key of a double
   unsigned long long u = (unsigned long long)__double_as_longlong(v);
   return (u >> 63) ? ~u : (u | 0x8000000000000000ULL);
 }
 __device__ __forceinline__ double okey_inv(unsigned long long k) {
-  unsigned long long u = (k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFULL) : ~k;
+  unsigned long long u = (k >> 63) ? (k & 0x7fffffffffffffffULL) : ~k;
   return __longlong_as_double((long long)u);
 }
 
+constexpr int MED_LIST = 256;  // candidates that are selected by counting (the square of their number)
 
-// the range and NaN of a warp's energies (a thread's smallest and largest key, ~0 and 0 without one) into the state: an
-// atomic only where it improves what is there already
-__device__ __forceinline__ void energy_range(EnergyStats::Half* h, unsigned long long lo, unsigned long long hi, bool nan) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
-    lo = a < lo ? a : lo;
-    hi = b > hi ? b : hi;
-  }
-  nan = __any_sync(0xffffffffu, nan);
-  if ((threadIdx.x & 31) == 0) {
-    if (lo < __ldcg(&h->lo)) atomicMin(&h->lo, lo);
-    if (hi > __ldcg(&h->hi)) atomicMax(&h->hi, hi);
-    if (nan) atomicOr(&h->nan, 1u);
-  }
+__device__ __forceinline__ EnergyStats::Half median_start() {
+  EnergyStats::Half h{};
+  h.lo = h.first = ~0ull;
+  return h;
 }
-
-// ---------------------------------------------------------------- energy median and reset
-// The median of the energy (np.median, phaseflow.py:149-151) by an exact radix select over order-preserving keys, and the
-// reset that reads it, in one cooperative launch whose blocks meet at grid barriers:
-// 1. the range of the energies (barrier) and the reset rule (phaseflow.rs:846-854): when every energy is above
-//    1e-9 max + 1e-30 no pixel is reset, and unless the caller needs the median every block returns.
-// 2. a histogram of 4096 equal parts of the keys' range (barrier), from which every block picks the median's part;
-// 3. the elements of that part into a candidate list (room for all n) and the largest key below it (barrier);
-// 4. every block selects the median among the candidates (by counting where there are at most 1024, else by 12-bit
-//    digits) and resets its share of the pixels.
-// Small images are bound by the launches' latency, large ones by the scans. Five launches before (two histogram scans, the
-// compaction, the final select, the reset; 80 per refinement): 128^2 pairs 1.459 -> 1.214 ms, 2048^2 30.85 -> 30.36 ms.
-// Taking the range in the solve's epilogue saves the first scan and barrier but costs the solve registers (2048^2: 0.333
-// -> 0.357 ms per launch), more than it gives. A barrier gives up after MED_SPINS polls, the median is NaN then.
-// threads, parts, energies a thread keeps in registers (4: 1.257 ms per 128^2 pair, 16: 1.285, 8: 1.214), and the energies
-// per block below one block per SM
-constexpr int MED_T = 1024, MED_BINS = 4096, MED_E = 8, MED_PER = MED_T * MED_E;
-constexpr unsigned MED_SPINS = 1u << 22;
-
 __global__ void k_stats_init(EnergyStats* s) {
   s->median = 0.0;
-  s->timeouts = 0;
-  for (int i = 0; i < 2; i++) s->half[i] = EnergyStats::Half{~0ull, 0ull, 0ull, 0u, 0u, 0u};
+  for (int i = 0; i < 2; i++) s->half[i] = median_start();
 }
 
-// every block of the grid arrives for the `round`-th time; false where the wait gave up
-__device__ bool grid_meet(EnergyStats* s, EnergyStats::Half* h, unsigned round) {
-  if (gridDim.x == 1) {
-    __syncthreads();
-    return true;
+// every energy is above 1e-9 max + 1e-30 (lo, hi: the smallest and largest key, ~0 and 0 where all are NaN)
+__device__ __forceinline__ bool median_skips(unsigned long long lo, unsigned long long hi, bool nan) {
+  const double vlo = okey_inv(lo), vhi = okey_inv(hi);
+  return !nan && vhi <= DBL_MAX / 2 && vlo > 1e-9 * vhi + 1e-30;
+}
+// log2 of the keys per part where [lo, hi] is split into at most 2^log_bins parts
+__device__ __forceinline__ int median_shift(unsigned long long lo, unsigned long long hi, int log_bins) {
+  return max(64 - __clzll((long long)(hi - lo)) - log_bins, 0);
+}
+__device__ __forceinline__ unsigned long long warp_max64(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w > v ? w : v;
   }
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&h->bar, 1u);
-    const unsigned want = round * gridDim.x;
-    unsigned seen = 0, k = 0;
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&h->bar) : "memory");
-    } while (seen < want && ++k < MED_SPINS);
-    ok = seen >= want;
-    if (seen < want) atomicAdd(&s->timeouts, 1u);
-    __threadfence();
-  }
-  __syncthreads();
-  return ok != 0;
+  return v;
 }
 
-// the bin of 4096 counts (count(i)) that holds `rank`, and the number of elements in the bins before it; every thread of
-// the block gets both. total: at least rank + 1
-template <class Count>
-__device__ void block_pick(Count count, long long rank, int& bin, long long& before) {
-  constexpr int PER = MED_BINS / MED_T;
-  __shared__ long long wsum[MED_T / 32], sh_before;
+// f(energy, index) for the thread's energies, the pairs i0, i0 + step, ... of n: the first E pairs, which the caller loaded
+// into v, from registers, later ones from memory, four loads at a time. e: 16-byte aligned
+template <class I>
+__device__ __forceinline__ double2 load_pair(const double* __restrict__ e, I n, I i) {
+  if (2 * i + 1 < n) return *reinterpret_cast<const double2*>(e + 2 * i);
+  return make_double2(2 * i < n ? e[2 * i] : 0.0, 0.0);
+}
+template <int E, class I>
+__device__ __forceinline__ void load_energies(const double* __restrict__ e, I n, I i0, I step, double2 (&v)[E]) {
+#pragma unroll
+  for (int u = 0; u < E; u++) v[u] = load_pair(e, n, i0 + u * step);
+}
+template <int E, class I, class F>
+__device__ __forceinline__ void each_energy(const double* __restrict__ e, I n, I i0, I step, const double2 (&v)[E], F f) {
+  auto both = [&](double2 w, I i) {
+    if (2 * i < n) f(w.x, 2 * i);
+    if (2 * i + 1 < n) f(w.y, 2 * i + 1);
+  };
+#pragma unroll
+  for (int u = 0; u < E; u++) both(v[u], i0 + u * step);
+  for (I i = i0 + E * step; 2 * i < n; i += 4 * step) {
+    double2 w[4];
+    load_energies(e, n, i, step, w);
+#pragma unroll
+    for (int u = 0; u < 4; u++) both(w[u], i + u * step);
+  }
+}
+
+// the smallest and largest key of a block's energies and whether one is NaN, into shared memory (~0, 0 and 0 before). The
+// caller synchronises
+template <int E, class I>
+__device__ __forceinline__ void energy_range(const double* __restrict__ e, I n, I i0, I step, const double2 (&v)[E],
+                                             unsigned long long* slo, unsigned long long* shi, unsigned* snan) {
+  unsigned long long lo = ~0ull, hi = 0;
+  bool nan = false;
+  each_energy(e, n, i0, step, v, [&](double x, auto) {
+    if (x != x) {
+      nan = true;
+    } else {
+      const unsigned long long k = okey(x);
+      lo = k < lo ? k : lo;
+      hi = k > hi ? k : hi;
+    }
+  });
+  __syncwarp();
+  lo = ~warp_max64(~lo);
+  hi = warp_max64(hi);
+  nan = __any_sync(0xffffffffu, nan);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(slo, lo);
+    atomicMax(shi, hi);
+    if (nan) atomicOr(snan, 1u);
+  }
+}
+
+// inclusive sums of v over the threads of a block of T; tot: T / 32 values of shared memory, the last of which holds the
+// sum over the block afterwards. The caller synchronises before tot is used again
+template <int T>
+__device__ long long block_scan(long long v, long long* tot) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long w = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += w;
+  }
+  if (lane == 31) tot[wid] = v;
+  __syncthreads();
+  if (wid == 0) {
+    long long w = lane < T / 32 ? tot[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    if (lane < T / 32) tot[lane] = w;
+  }
+  __syncthreads();
+  return v + (wid ? tot[wid - 1] : 0);
+}
+
+// the bin of BINS counts (count(i)) that holds `rank`, the number of elements in the bins before it and its own; every
+// thread of the block of T gets them. The counts sum to more than rank
+template <int T, int BINS, class Count>
+__device__ void block_pick(Count count, long long rank, int& bin, long long& before, unsigned& in) {
+  constexpr int PER = BINS / T;
+  __shared__ long long tot[T / 32], sh_before;
   __shared__ int sh_bin;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  __shared__ unsigned sh_in;
   unsigned c[PER];
   long long loc = 0;
 #pragma unroll
   for (int j = 0; j < PER; j++) {
-    c[j] = count(tid * PER + j);
+    c[j] = count((int)threadIdx.x * PER + j);
     loc += c[j];
   }
-  long long inc = loc;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const long long v = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += v;
-  }
-  if (lane == 31) wsum[wid] = inc;
-  __syncthreads();
-  if (wid == 0) {
-    long long w = wsum[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long v = __shfl_up_sync(0xffffffffu, w, o);
-      if (lane >= o) w += v;
-    }
-    wsum[lane] = w;
-  }
-  __syncthreads();
-  long long acc = inc - loc + (wid ? wsum[wid - 1] : 0);
+  long long acc = block_scan<T>(loc, tot) - loc;
   if (acc <= rank && rank < acc + loc) {  // exactly one thread
-    int j = 0;
+    bool found = false;
 #pragma unroll
-    for (int i = 0; i < PER - 1; i++)
-      if (j == i && acc + c[i] <= rank) {
-        acc += c[i];
-        j = i + 1;
+    for (int j = 0; j < PER; j++) {
+      if (!found && rank < acc + c[j]) {
+        found = true;
+        sh_bin = (int)threadIdx.x * PER + j;
+        sh_before = acc;
+        sh_in = c[j];
       }
-    sh_bin = tid * PER + j;
-    sh_before = acc;
+      if (!found) acc += c[j];
+    }
   }
   __syncthreads();
   bin = sh_bin;
   before = sh_before;
+  in = sh_in;
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(MED_T) k_median_reset(const double* __restrict__ e, size_t n, EnergyStats* s, int half,
-                                                      int force, unsigned* hist2, unsigned long long* cand,
-                                                      const double* __restrict__ uxin, const double* __restrict__ uyin,
-                                                      double* ux, double* uy, double* resid, double* slope) {
-  __shared__ unsigned h[MED_BINS];
-  __shared__ unsigned long long keys[MED_T];
-  __shared__ unsigned long long sh_key, sh_below;
+// the key of rank `rank` among the nc <= MED_LIST keys (shared memory) by counting, and how many of them are less; every
+// thread of the block gets both. nc > rank
+__device__ void count_select(const unsigned long long* keys, unsigned nc, long long rank, unsigned long long& key,
+                             long long& less) {
+  __shared__ unsigned long long sh_key;
   __shared__ long long sh_less;
-  EnergyStats::Half& P = s->half[half];
-  unsigned* hist = hist2 + half * MED_BINS;
-  const int tid = threadIdx.x, lane = tid & 31;
-  const size_t i0 = blockIdx.x * (size_t)MED_T + tid, step = (size_t)gridDim.x * MED_T;
-  unsigned round = 0;
-  // the other half's start state for the next solve and median (the launch that used it has ended)
-  for (size_t i = i0; i < MED_BINS; i += step) hist2[(half ^ 1) * MED_BINS + i] = 0;
-  if (i0 == 0) s->half[half ^ 1] = EnergyStats::Half{~0ull, 0ull, 0ull, 0u, 0u, 0u};
-  // a thread's first MED_E energies stay in registers (all of them up to MED_T MED_E per block), later ones are read again
-  double v[MED_E];
-#pragma unroll
-  for (int u = 0; u < MED_E; u++) v[u] = i0 + u * step < n ? e[i0 + u * step] : 0.0;
-  auto each = [&](auto f) {
-#pragma unroll
-    for (int u = 0; u < MED_E; u++)
-      if (i0 + u * step < n) f(v[u], i0 + u * step);
-    for (size_t i = i0 + MED_E * step; i < n; i += 4 * step) {
-      double w[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) w[u] = i + u * step < n ? e[i + u * step] : 0.0;
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (i + u * step < n) f(w[u], i + u * step);
+  for (unsigned t = threadIdx.x; t < nc; t += blockDim.x) {
+    const unsigned long long k = keys[t];
+    unsigned lt = 0, le = 0;
+    for (unsigned i = 0; i < nc; i++) {
+      lt += keys[i] < k;
+      le += keys[i] <= k;
     }
-  };
-  // 1. the range of the energies
-  {
-    unsigned long long lo = ~0ull, hi = 0;
-    bool nan = false;
-    each([&](double x, size_t) {
-      if (x != x) {
-        nan = true;
-      } else {
-        const unsigned long long k = okey(x);
-        lo = k < lo ? k : lo;
-        hi = k > hi ? k : hi;
-      }
-    });
-    __syncwarp();
-    energy_range(&P, lo, hi, nan);
-    if (!grid_meet(s, &P, ++round)) return;
+    if ((long long)lt <= rank && rank < (long long)le) {  // the equal keys of that rank write the same values
+      sh_key = k;
+      sh_less = lt;
+    }
   }
-  const unsigned long long klo = __ldcg(&P.lo), khi = __ldcg(&P.hi);
-  const bool nan = __ldcg(&P.nan) != 0;
-  // the reset needs the median unless every energy is above 1e-9 max + 1e-30 (phaseflow.rs:846-854)
-  const double vlo = okey_inv(klo), vhi = okey_inv(khi);
-  const bool skip = !nan && vhi <= DBL_MAX / 2 && vlo > 1e-9 * vhi + 1e-30;
+  __syncthreads();
+  key = sh_key;
+  less = sh_less;
+}
+
+// the largest of the nc keys at(i) below `key`, or `floor` if that is larger; every thread of the block gets it
+template <class At>
+__device__ unsigned long long block_below(At at, unsigned nc, unsigned long long key, unsigned long long floor) {
+  __shared__ unsigned long long sh;
+  if (threadIdx.x == 0) sh = floor;
+  __syncthreads();
+  unsigned long long best = 0;
+  for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) {
+    const unsigned long long k = at(i);
+    if (k < key && k > best) best = k;
+  }
+  __syncwarp();
+  best = warp_max64(best);
+  if ((threadIdx.x & 31) == 0 && best) atomicMax(&sh, best);
+  __syncthreads();
+  return sh;
+}
+
+struct ResetPlanes {  // the planes of the reset; ux null: none
+  const double *uxin, *uyin;
+  double *ux, *uy, *resid, *slope;
+};
+__device__ __forceinline__ void reset_pixel(const ResetPlanes& r, size_t n, size_t p) {
+  r.ux[p] = r.uxin[p];
+  r.uy[p] = r.uyin[p];
+  r.resid[p] = PI;
+  for (int i = 0; i < 4; i++) r.slope[i * n + p] = 0.0;
+}
+
+// ---- one cluster: the steps' results in the blocks' shared memory
+constexpr int MC_B = 8, MC_T = 512, MC_E = 4;  // blocks, threads, pairs of energies a thread keeps in registers
+constexpr int MC_LOG = 12, MC_BINS = 1 << MC_LOG;  // parts of a histogram
+static_assert(MC_BINS == MC_B * MC_T, "a bin per thread of the cluster");
+
+__global__ void __cluster_dims__(MC_B, 1, 1) __launch_bounds__(MC_T, 2)
+    k_median_cluster(const double* __restrict__ e, unsigned n, EnergyStats* s, int force, ResetPlanes rp) {
+  grid_dep_wait();
+  namespace cg = cooperative_groups;
+  __shared__ unsigned h[MC_BINS];
+  __shared__ unsigned long long keys[MED_LIST];
+  __shared__ unsigned long long lo, hi, below, all_lo, all_hi, all_below;
+  __shared__ unsigned nan, ncand;
+  __shared__ bool all_nan;
+  __shared__ long long tot[MC_T / 32], sh_before;
+  __shared__ int sh_bin;
+  __shared__ unsigned sh_in;
+  const cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, rank_b = (int)cl.block_rank();
+  const unsigned i0 = rank_b * MC_T + tid, step = MC_B * MC_T;
+  double2 v[MC_E];
+  load_energies(e, n, i0, step, v);
+  if (tid == 0) {
+    lo = ~0ull;
+    hi = below = 0;
+    nan = ncand = 0;
+  }
+  for (int i = tid; i < MC_BINS; i += MC_T) h[i] = 0;
+  __syncthreads();
+  energy_range(e, n, i0, step, v, &lo, &hi, &nan);
+  cl.sync();
+  if (tid < 32) {  // a block's range per lane
+    const int b = tid % MC_B;
+    const unsigned long long l = ~warp_max64(~*cl.map_shared_rank(&lo, b)), m = warp_max64(*cl.map_shared_rank(&hi, b));
+    const bool any = __any_sync(0xffffffffu, *cl.map_shared_rank(&nan, b) != 0);
+    if (tid == 0) {
+      all_lo = l;
+      all_hi = m;
+      all_nan = any;
+    }
+  }
+  cl.sync();  // the blocks' ranges are read
+  const unsigned long long klo = all_lo, khi = all_hi;
+  const bool skip = median_skips(klo, khi, all_nan);
   if (!force && skip) return;
   double med = ::nan("");
-  if (!nan) {
-    // 2. the part of the range that holds the element of rank n / 2
-    const unsigned long long range = khi - klo;
-    const int bits = 64 - __clzll((long long)range), shift = bits > 12 ? bits - 12 : 0;
-    for (int i = tid; i < MED_BINS; i += MED_T) h[i] = 0;
-    __syncthreads();
-    each([&](double x, size_t) { atomicAdd(&h[(okey(x) - klo) >> shift], 1u); });
-    __syncthreads();
-    for (int i = tid; i < MED_BINS; i += MED_T)
-      if (h[i]) atomicAdd(&hist[i], h[i]);
-    if (!grid_meet(s, &P, ++round)) {
-      if (i0 == 0) s->median = med;
-      return;
+  if (!all_nan) {
+    long long rank = n / 2, less = 0;
+    unsigned long long base = klo, width = khi - klo;  // keys of the part: base .. base + width
+    for (int shift = median_shift(klo, khi, MC_LOG);; shift = max(shift - MC_LOG, 0)) {
+      each_energy(e, n, i0, step, v, [&](double x, auto) {
+        const unsigned long long k = okey(x) - base;  // below base: beyond any width
+        if (k <= width) atomicAdd(&h[k >> shift], 1u);
+      });
+      cl.sync();
+      // a bin per thread of the cluster: the sums over the blocks, the block's share of the ranks
+      unsigned c = 0;
+#pragma unroll
+      for (int b = 0; b < MC_B; b++) c += cl.map_shared_rank(h, b)[rank_b * MC_T + tid];
+      long long excl = block_scan<MC_T>(c, tot) - c;
+      cl.sync();
+#pragma unroll 1
+      for (int b = 0; b < rank_b; b++) excl += cl.map_shared_rank(tot, b)[MC_T / 32 - 1];
+      if (excl <= rank && rank < excl + c) {  // exactly one thread of the cluster
+#pragma unroll 1
+        for (int b = 0; b < MC_B; b++) {
+          *cl.map_shared_rank(&sh_bin, b) = rank_b * MC_T + tid;
+          *cl.map_shared_rank(&sh_before, b) = excl;
+          *cl.map_shared_rank(&sh_in, b) = c;
+        }
+      }
+      for (int i = tid; i < MC_BINS; i += MC_T) h[i] = 0;  // its readers have met
+      cl.sync();
+      base += (unsigned long long)sh_bin << shift;
+      width = (1ull << shift) - 1;
+      rank -= sh_before;
+      less += sh_before;
+      if (shift == 0 || sh_in <= MED_LIST) break;
     }
-    long long rank = (long long)(n / 2), less = 0, before;
-    int bin;
-    block_pick([&](int i) { return __ldcg(hist + i); }, rank, bin, before);
-    rank -= before;
-    less += before;
-    // 3. that part's elements, and the largest key below it
-    const unsigned long long base = klo + ((unsigned long long)bin << shift);
-    const unsigned long long width = 1ull << shift;  // keys of the part: [base, base + width)
-    unsigned long long below = 0;
-    each([&](double x, size_t) {
+    // the part's elements into block 0's list (where its keys differ), and the largest key below the part
+    const bool list = width > 0;
+    unsigned* count = cl.map_shared_rank(&ncand, 0);
+    unsigned long long *cand = cl.map_shared_rank(keys, 0), under = 0;
+    each_energy(e, n, i0, step, v, [&](double x, auto) {
       const unsigned long long k = okey(x);
-      if (k < base) below = k > below ? k : below;
-      else if (k - base < width) cand[atomicAdd(&P.ncand, 1u)] = k;  // the active lanes' additions are made as one
+      if (k < base) under = k > under ? k : under;
+      else if (list && k - base <= width) cand[atomicAdd(count, 1u)] = k;
     });
     __syncwarp();
-    for (int o = 16; o; o >>= 1) {
-      const unsigned long long v = __shfl_xor_sync(0xffffffffu, below, o);
-      below = v > below ? v : below;
+    under = warp_max64(under);
+    if ((tid & 31) == 0 && under) atomicMax(&below, under);
+    cl.sync();
+    const unsigned nc = *count;
+    if (tid < 32) {
+      under = warp_max64(*cl.map_shared_rank(&below, tid % MC_B));
+      if (tid == 0) all_below = under;
     }
-    if (lane == 0 && below > __ldcg(&P.below)) atomicMax(&P.below, below);
-    if (!grid_meet(s, &P, ++round)) {
-      if (i0 == 0) s->median = med;
-      return;
+    if (rank_b > 0)
+      for (unsigned i = tid; i < nc; i += MC_T) keys[i] = cand[i];
+    cl.sync();  // block 0 may end, and every block's own copy is whole
+    unsigned long long kmed = base;
+    if (list) {
+      long long lt;
+      count_select(keys, nc, rank, kmed, lt);
+      less += lt;
     }
-    // 4. the element of that rank among the candidates
-    const unsigned nc = __ldcg(&P.ncand);
-    if (tid == 0) sh_below = __ldcg(&P.below);
-    if (nc <= MED_T) {
-      const unsigned long long key = (unsigned)tid < nc ? __ldcg(cand + tid) : ~0ull;
-      keys[tid] = key;
-      __syncthreads();
-      if ((unsigned)tid < nc) {
-        unsigned lt = 0, le = 0;
-        for (unsigned i = 0; i < nc; i++) {
-          lt += keys[i] < key;
-          le += keys[i] <= key;
-        }
-        if ((long long)lt <= rank && rank < (long long)le) {  // the equal keys of that rank write the same values
-          sh_key = key;
-          sh_less = less + lt;
-        }
-      }
-      __syncthreads();
-    } else {
-      unsigned long long prefix = 0;  // the digits fixed so far of key - base
-      for (int rem = shift; rem > 0;) {
-        const int d = rem < 12 ? rem : 12, sh = rem - d;
-        for (int i = tid; i < MED_BINS; i += MED_T) h[i] = 0;
-        __syncthreads();
-        for (unsigned i = tid; i < nc; i += MED_T) {
-          const unsigned long long k = __ldcg(cand + i) - base;
-          if ((k >> rem) == prefix) atomicAdd(&h[(k >> sh) & ((1u << d) - 1)], 1u);
-        }
-        __syncthreads();
-        block_pick([&](int i) { return h[i]; }, rank, bin, before);
-        rank -= before;
-        less += before;
-        prefix = (prefix << d) | (unsigned)bin;
-        rem = sh;
-      }
-      if (tid == 0) {
-        sh_key = base + prefix;
-        sh_less = less;
-      }
-      __syncthreads();
-    }
-    const unsigned long long kmed = sh_key;
     med = okey_inv(kmed);
     // an even count's lower middle: the same value unless exactly n / 2 elements are below it, then the largest of those
-    if (n % 2 == 0 && sh_less >= (long long)(n / 2)) {
-      unsigned long long best = 0;
-      for (unsigned i = tid; i < nc; i += MED_T) {
-        const unsigned long long k = __ldcg(cand + i);
-        if (k < kmed && k > best) best = k;
-      }
-      for (int o = 16; o; o >>= 1) {
-        const unsigned long long v = __shfl_xor_sync(0xffffffffu, best, o);
-        best = v > best ? v : best;
-      }
-      if (lane == 0 && best) atomicMax(&sh_below, best);
-      __syncthreads();
-      med = (okey_inv(sh_below) + med) / 2.0;
-    }
+    if (n % 2 == 0 && less >= (long long)(n / 2)) med = (okey_inv(block_below([&](unsigned i) { return keys[i]; }, nc, kmed, all_below)) + med) / 2.0;
   }
   if (i0 == 0) s->median = med;
-  if (skip || !ux) return;
+  if (skip || !rp.ux) return;
   const double thr = 1e-9 * med + 1e-30;
-  each([&](double x, size_t p) {
-    if (!(x > thr)) {
-      ux[p] = uxin[p];
-      uy[p] = uyin[p];
-      resid[p] = PI;
-      for (int i = 0; i < 4; i++) slope[(size_t)i * n + p] = 0.0;
+  each_energy(e, n, i0, step, v, [&](double x, unsigned p) {
+    if (!(x > thr)) reset_pixel(rp, n, p);
+  });
+}
+
+// ---- a launch per step
+constexpr int ML_T = 512, ML_E = 2;  // threads, pairs of energies a thread keeps in registers
+// blocks of a scan: a thread's first ML_E pairs cover n, at most two blocks per SM of 148
+static unsigned median_blocks(size_t n) { return std::min(296u, div_up(n, 2 * ML_T * ML_E)); }
+
+// whether this is the last block of the grid to arrive (its writes before are visible to that block); every thread gets it
+__device__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+__global__ void __launch_bounds__(ML_T, 2) k_median_range(const double* __restrict__ e, size_t n, EnergyStats* s, int half) {
+  grid_dep_wait();
+  const size_t i0 = blockIdx.x * (size_t)ML_T + threadIdx.x, step = (size_t)gridDim.x * ML_T;
+  // the other half's start state for the next median (the launches that used it have ended)
+  if (i0 == 0) s->half[half ^ 1] = median_start();
+  EnergyStats::Half& P = s->half[half];
+  __shared__ unsigned long long lo, hi;
+  __shared__ unsigned nan;
+  double2 v[ML_E];
+  load_energies(e, n, i0, step, v);
+  if (threadIdx.x == 0) {
+    lo = ~0ull;
+    hi = 0;
+    nan = 0;
+  }
+  __syncthreads();
+  energy_range(e, n, i0, step, v, &lo, &hi, &nan);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicMin(&P.lo, lo);
+    atomicMax(&P.hi, hi);
+    if (nan) atomicOr(&P.nan, 1u);
+  }
+}
+
+constexpr int ML_LOG = 12, ML_BINS = 1 << ML_LOG;  // parts of a histogram
+// the median is not needed
+__device__ __forceinline__ bool median_done(const EnergyStats::Half& P, int force) {
+  return !force && median_skips(P.lo, P.hi, P.nan != 0);
+}
+
+// the last block picks the part and leaves the histogram zero
+__global__ void __launch_bounds__(ML_T, 2) k_median_hist(const double* __restrict__ e, size_t n, EnergyStats* s, int half,
+                                                       int force, unsigned* hist) {
+  grid_dep_wait();
+  EnergyStats::Half& P = s->half[half];
+  if (P.nan || median_done(P, force)) return;
+  __shared__ unsigned h[ML_BINS];
+  const unsigned long long base = P.lo;
+  const int shift = median_shift(P.lo, P.hi, ML_LOG);
+  const size_t i0 = blockIdx.x * (size_t)ML_T + threadIdx.x, step = (size_t)gridDim.x * ML_T;
+  double2 v[ML_E];
+  load_energies(e, n, i0, step, v);
+  for (int i = threadIdx.x; i < ML_BINS; i += ML_T) h[i] = 0;
+  __syncthreads();
+  each_energy(e, n, i0, step, v, [&](double x, auto) { atomicAdd(&h[(okey(x) - base) >> shift], 1u); });
+  __syncthreads();
+  for (int i = threadIdx.x; i < ML_BINS; i += ML_T)
+    if (h[i]) atomicAdd(&hist[i], h[i]);
+  if (!last_block(&P.ticket)) return;
+  int bin;
+  long long before;
+  unsigned in;
+  block_pick<ML_T, ML_BINS>([&](int i) { return __ldcg(hist + i); }, (long long)(n / 2), bin, before, in);
+  for (int i = threadIdx.x; i < ML_BINS; i += ML_T) hist[i] = 0;
+  if (threadIdx.x == 0) {
+    P.base = base + ((unsigned long long)bin << shift);
+    P.less = before;
+    P.shift = shift;
+  }
+}
+
+// the part's elements as a list, the largest key below the part; the last block selects the median
+__global__ void __launch_bounds__(ML_T, 2) k_median_select(const double* __restrict__ e, size_t n, EnergyStats* s, int half,
+                                                         int force, unsigned long long* cand) {
+  grid_dep_wait();
+  EnergyStats::Half& P = s->half[half];
+  if (median_done(P, force)) return;
+  if (P.nan) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) s->median = nan("");
+    return;
+  }
+  __shared__ unsigned h[ML_BINS];
+  __shared__ unsigned long long keys[MED_LIST], below, first, last;
+  __shared__ unsigned nkeys;
+  const unsigned long long base = P.base, width = (1ull << P.shift) - 1;
+  const size_t i0 = blockIdx.x * (size_t)ML_T + threadIdx.x, step = (size_t)gridDim.x * ML_T;
+  double2 v[ML_E];
+  load_energies(e, n, i0, step, v);
+  if (threadIdx.x == 0) {
+    below = last = 0;
+    first = ~0ull;
+    nkeys = 0;
+  }
+  __syncthreads();
+  unsigned long long under = 0, lo = ~0ull, hi = 0;
+  each_energy(e, n, i0, step, v, [&](double x, auto) {
+    const unsigned long long k = okey(x);
+    if (k < base) {
+      under = k > under ? k : under;
+    } else if (k - base <= width) {
+      lo = k < lo ? k : lo;
+      hi = k > hi ? k : hi;
+      cand[atomicAdd(&P.ncand, 1u)] = k;  // the active lanes' additions are made as one
     }
+  });
+  __syncwarp();
+  under = warp_max64(under);
+  lo = ~warp_max64(~lo);
+  hi = warp_max64(hi);
+  if ((threadIdx.x & 31) == 0) {
+    if (under) atomicMax(&below, under);
+    if (hi) {
+      atomicMin(&first, lo);
+      atomicMax(&last, hi);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (below) atomicMax(&P.below, below);
+    if (last) {
+      atomicMin(&P.first, first);
+      atomicMax(&P.last, last);
+    }
+  }
+  if (!last_block(&P.ticket)) return;
+  const unsigned nc = __ldcg(&P.ncand);
+  // f(key) for the candidates from lo to hi
+  auto among = [&](auto f) {
+    for (unsigned i = threadIdx.x; i < nc; i += 8 * ML_T) {
+      unsigned long long k[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) k[u] = i + u * ML_T < nc ? __ldcg(cand + i + u * ML_T) : ~0ull;
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        if (k[u] - lo <= hi - lo) f(k[u]);
+    }
+  };
+  lo = __ldcg(&P.first);
+  hi = __ldcg(&P.last);
+  long long less = P.less, rank = (long long)(n / 2) - less;
+  for (unsigned in = nc; in > MED_LIST && lo != hi;) {  // the candidates' range split again
+    const int shift = median_shift(lo, hi, ML_LOG);
+    for (int i = threadIdx.x; i < ML_BINS; i += ML_T) h[i] = 0;
+    __syncthreads();
+    among([&](unsigned long long k) { atomicAdd(&h[(k - lo) >> shift], 1u); });
+    __syncthreads();
+    int bin;
+    long long before;
+    block_pick<ML_T, ML_BINS>([&](int i) { return h[i]; }, rank, bin, before, in);
+    rank -= before;
+    less += before;
+    lo += (unsigned long long)bin << shift;
+    hi = min(hi, lo + ((1ull << shift) - 1));
+  }
+  unsigned long long kmed = lo;
+  if (lo != hi) {
+    among([&](unsigned long long k) { keys[atomicAdd(&nkeys, 1u)] = k; });
+    __syncthreads();
+    long long lt;
+    count_select(keys, nkeys, rank, kmed, lt);
+    less += lt;
+  }
+  double med = okey_inv(kmed);
+  // an even count's lower middle: the same value unless exactly n / 2 elements are below it, then the largest of those
+  if (n % 2 == 0 && less >= (long long)(n / 2))
+    med = (okey_inv(block_below([&](unsigned i) { return __ldcg(cand + i); }, nc, kmed, __ldcg(&P.below))) + med) / 2.0;
+  if (threadIdx.x == 0) s->median = med;
+}
+
+__global__ void __launch_bounds__(ML_T, 2) k_median_reset(const double* __restrict__ e, size_t n, const EnergyStats* s, int half,
+                                                        ResetPlanes rp) {
+  grid_dep_wait();
+  const EnergyStats::Half& P = s->half[half];
+  if (median_skips(P.lo, P.hi, P.nan != 0)) return;
+  const double thr = 1e-9 * s->median + 1e-30;
+  const size_t i0 = blockIdx.x * (size_t)ML_T + threadIdx.x, step = (size_t)gridDim.x * ML_T;
+  double2 v[ML_E];
+  load_energies(e, n, i0, step, v);
+  each_energy(e, n, i0, step, v, [&](double x, size_t p) {
+    if (!(x > thr)) reset_pixel(rp, n, p);
   });
 }
 
 void launch_energy_stats_init(EnergyStats* stats, unsigned long long* scratch, cudaStream_t st) {
-  OFC_CUDA(cudaMemsetAsync(scratch, 0, 2 * MED_BINS * sizeof(unsigned), st));
+  OFC_CUDA(cudaMemsetAsync(scratch, 0, ML_BINS * sizeof(unsigned), st));
   OFC_LAUNCH(k_stats_init, 1, 1, 0, st, stats);
 }
 
 void launch_median_reset(const double* energy, size_t n, EnergyStats* stats, int half, bool force,
                          unsigned long long* scratch, const double* ux_in, const double* uy_in, double* ux, double* uy,
                          double* resid, double* slope, cudaStream_t st) {
-  int dev = 0, sms = 0;
-  OFC_CUDA(cudaGetDevice(&dev));
-  OFC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // one block per SM at most: every block is resident in a cooperative launch
-  const int grid = (int)std::min<size_t>((size_t)sms, std::max<size_t>(1, n / MED_PER));
+  const ResetPlanes rp{ux_in, uy_in, ux, uy, resid, slope};
+  const int f = force ? 1 : 0;
+  if (n <= MED_CLUSTER_N) {
+    OFC_LAUNCH_PDL(k_median_cluster, MC_B, MC_T, 0, st, energy, (unsigned)n, stats, f, rp);
+    return;
+  }
+  const unsigned g = median_blocks(n);
+  OFC_LAUNCH_PDL(k_median_range, g, ML_T, 0, st, energy, n, stats, half);
   unsigned* hist = (unsigned*)scratch;
-  unsigned long long* cand = scratch + MED_BINS;  // after the two histograms
-  int f = force;
-  void* args[] = {&energy, &n, &stats, &half, &f, &hist, &cand, &ux_in, &uy_in, &ux, &uy, &resid, &slope};
-  void* tok = nullptr;
-  if (g_profiler) prof_before("k_median_reset", st, &tok);
-  OFC_CUDA(cudaLaunchCooperativeKernel((const void*)k_median_reset, dim3(grid), dim3(MED_T), args, 0, st));
-  if (tok) prof_after(tok, st);
-  if (g_launch_counter) ++*g_launch_counter;
+  unsigned long long* cand = scratch + ML_BINS / 2;  // after the histogram
+  OFC_LAUNCH_PDL(k_median_hist, g, ML_T, 0, st, energy, n, stats, half, f, hist);
+  OFC_LAUNCH_PDL(k_median_select, g, ML_T, 0, st, energy, n, stats, half, f, cand);
+  if (ux) OFC_LAUNCH_PDL(k_median_reset, g, ML_T, 0, st, energy, n, stats, half, rp);
 }
 
 // ---------------------------------------------------------------- confidence

@@ -61,22 +61,24 @@ void launch_moments_solve(const double* sums, const double* ux, const double* uy
 // for the next.
 struct EnergyStats {
   double median;
-  unsigned timeouts;  // grid barriers that gave up (the median is NaN then)
   struct Half {
     unsigned long long lo, hi;  // the smallest and largest energy as order-preserving keys (~0 and 0: none yet)
-    unsigned long long below;   // the largest key below the median's bucket
+    unsigned long long below;   // the largest key below the picked part
+    unsigned long long first, last;  // the smallest and largest key of the part
+    unsigned long long base;    // the part's keys: base .. base + 2^shift - 1
+    long long less;             // elements below the part
     unsigned nan;               // an energy is NaN
-    unsigned ncand;             // elements in the median's bucket
-    unsigned bar;               // arrivals at the grid barriers
+    unsigned ncand;             // elements of the part
+    unsigned ticket;            // blocks of the running launch that are done
+    int shift;
   } half[2];
 };
-// unsigned long long of the median's scratch for n energies: two histograms of 4096 counts, then up to n candidates
-inline size_t median_scratch(size_t n) { return 4096 + n; }
-// the start state of both halves and zero histograms
+// unsigned long long of the median's scratch for n energies: a histogram of 4096 32-bit counts, then up to n candidates
+inline size_t median_scratch(size_t n) { return 2048 + n; }
+// the start state of both halves and a zero histogram
 void launch_energy_stats_init(EnergyStats* stats, unsigned long long* scratch, cudaStream_t st);
 // The reset below 1e-9 median + 1e-30 (phaseflow.py:149-151,158-161) of ux, uy, resid and slope (ux null: no reset) when an
-// energy needs it, and the median into stats->median (np.median) when the reset needs it or `force`, in one launch on
-// `half` of the state
+// energy needs it, and the median into stats->median (np.median) when the reset needs it or `force`, on `half` of the state
 void launch_median_reset(const double* energy, size_t n, EnergyStats* stats, int half, bool force,
                          unsigned long long* scratch, const double* ux_in, const double* uy_in, double* ux, double* uy,
                          double* resid, double* slope, cudaStream_t st);

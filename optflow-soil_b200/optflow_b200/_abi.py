@@ -225,6 +225,7 @@ TEST_SIGNATURES = {
     "ofc_test_local_solve": (ctypes.c_int, [_P, c_double_p, c_double_p, c_double_p, _S, _S, ctypes.POINTER(OfcConfig)]
                              + [c_double_p] * 5 + [_E, _S]),
     "ofc_test_median": (ctypes.c_int, [_P, c_double_p, _S, c_double_p, _E, _S]),
+    "ofc_test_median_reset": (ctypes.c_int, [_P, c_double_p, _S, _S, c_u8_p, c_double_p, c_double_p, c_double_p, _E, _S]),
     "ofc_test_large_components": (ctypes.c_int, [_P, c_u8_p, _S, _S, ctypes.c_double, c_u8_p, _E, _S]),
     "ofc_test_first_sums": (ctypes.c_int, [_P, c_float_p, c_float_p, _S, _S, c_double_p, c_double_p,
                                            ctypes.POINTER(OfcConfig), c_double_p, _E, _S]),

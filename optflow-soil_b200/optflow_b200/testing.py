@@ -68,6 +68,20 @@ def median(v, engine=None):
     return out.value
 
 
+def median_reset(energies, force, u, engine=None):
+    """Energy medians and resets one after the other on one state (ofc_test_median_reset): energies (rounds, n), force
+    (rounds,), u (2, n). Returns the medians and the planes (rounds, 7, n): ux, uy, resid, slope x 4."""
+    eng = engine or default_engine()
+    e, uu = _d(energies), _d(u)
+    rounds, n = e.shape
+    f = np.ascontiguousarray(force, dtype=np.uint8)
+    med = np.empty(rounds)
+    planes = np.empty((rounds, 7, n))
+    eng._call("ofc_test_median_reset", _ptr(e, c_double_p), rounds, n, _ptr(f, c_u8_p), _ptr(uu, c_double_p),
+              _ptr(med, c_double_p), _ptr(planes, c_double_p))
+    return med, planes
+
+
 def large_components(b, min_area, engine=None):
     eng = engine or default_engine()
     a = np.ascontiguousarray(b, dtype=np.uint8)

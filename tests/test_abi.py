@@ -140,3 +140,16 @@ def test_pixel_formats_and_save_result(tmp_path):
     assert np.load(tmp_path / "f1" / "valid.npy").tolist() == np.isfinite(ux).astype(np.uint8).tolist()
     assert np.load(tmp_path / "f1" / "fb.npy").dtype == np.dtype("<i4")
     assert json.load(open(tmp_path / "f1" / "timing.json")) == {"coarse": 0.1, "reference": 2}
+
+
+def test_no_launch_needs_the_whole_device():
+    """No kernel is launched cooperatively: a grid whose blocks wait for one another needs all of them resident at once,
+    which a device shared with other streams' kernels, or confined to fewer SMs, cannot promise."""
+    import glob
+    import os
+    csrc = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "optflow-soil_b200", "csrc")
+    files = glob.glob(os.path.join(csrc, "*.cu")) + glob.glob(os.path.join(csrc, "*.cuh"))
+    assert len(files) > 10
+    for f in files:
+        text = open(f).read()
+        assert "cudaLaunchCooperativeKernel" not in text and "cudaLaunchAttributeCooperative" not in text, f

@@ -268,6 +268,39 @@ def test_median_blocks_and_special_values(T, n):
     assert np.isnan(T.median(v))
 
 
+@pytest.mark.parametrize("n", [1, 2, 33, 4096, 65537, 98304, 98305, 303104, 606209, 1300001])
+def test_median_reset_rounds(T, n):
+    """Medians and resets in sequence on the alternating halves of one state, exactly: no pixel below the threshold (the
+    median needed or not), some far below it, energies over 80 decades, a NaN, ties, one value for half of them, one far
+    outlier on either side. Sizes around the cluster's limit, its registers and the launches' full grid, odd and even."""
+    rng = np.random.default_rng(n)
+    base = rng.exponential(size=n) + 0.1
+    few = base.copy()
+    few[rng.random(n) < 0.1] *= 1e-12
+    few[: n // 50] = 0.0
+    wide = base * 10.0 ** rng.uniform(-40, 40, n)
+    nan = few.copy()
+    nan[n // 2] = np.nan
+    ties = rng.integers(0, 3, n) * 1.0
+    half = np.where(rng.random(n) < 0.55, 0.0, base)
+    out1, out2 = base.copy(), base.copy()
+    out1[n // 3], out2[n // 3] = 1e-300, 1e300
+    rounds = [(base, 0), (few, 0), (few[::-1], 1), (base, 1), (wide, 0), (wide, 1), (nan, 0), (base, 0), (ties, 0), (half, 1),
+              (out1, 0), (out2, 1), (np.full(n, 0.25), 1), (few, 0)]
+    e = np.stack([v for v, _ in rounds])
+    u = rng.normal(size=(2, n))
+    med, planes = T.median_reset(e, [f for _, f in rounds], u)
+    for k, (v, force) in enumerate(rounds):
+        skip = not np.isnan(v).any() and v.min() > 1e-9 * v.max() + 1e-30
+        want = np.median(v)
+        if force or not skip:
+            np.testing.assert_equal(med[k], want, err_msg=str(k))
+        hit = np.zeros(n, bool) if skip else ~(v > 1e-9 * want + 1e-30)
+        np.testing.assert_array_equal(planes[k, :2], np.where(hit, u, 0.0), err_msg=str(k))
+        np.testing.assert_array_equal(planes[k, 2], np.where(hit, np.pi, 0.0), err_msg=str(k))
+        np.testing.assert_array_equal(planes[k, 3:], np.broadcast_to(np.where(hit, 0.0, np.nan), (4, n)), err_msg=str(k))
+
+
 def test_large_components(T, oracle):
     rng = np.random.default_rng(9)
     for p in (0.3, 0.5, 0.6):
