@@ -45,6 +45,10 @@ OFC_API int ofc_test_median(ofc_engine* eng, const double* v, size_t n, double* 
 OFC_API int ofc_test_median_reset(ofc_engine* eng, const double* energy, size_t rounds, size_t n, const uint8_t* force,
                                   const double* u, double* medians, double* planes, char* err, size_t errlen);
 
+/* Backs the host pages of [p, p + bytes) before they are written, their contents as they are (ofc_track_pairs does so with
+ * the planes of a pair that the GPU is working on). */
+OFC_API void ofc_test_populate(void* p, size_t bytes);
+
 /* track._large_components (python/optflow_ref/track.py:45-53) of a w x h mask. */
 OFC_API int ofc_test_large_components(ofc_engine* eng, const uint8_t* b, size_t w, size_t h, double min_area,
                                       uint8_t* out, char* err, size_t errlen);

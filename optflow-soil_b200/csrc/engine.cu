@@ -19,6 +19,9 @@
 #include <thread>
 #include <unordered_map>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include "fft.cuh"
 #include "synth_field.cuh"
 #include "kernels.cuh"
@@ -2147,6 +2150,27 @@ static void copy_pair_out(const ofc_pair_out& s, ofc_pair_out* d, size_t N) {
   for (int i = 0; i < 3; i++) d->timing[i] = s.timing[i];
 }
 
+// Has the kernel back the pages that hold [p, p + bytes) before they are written, their contents as they are; a hint, where
+// the system cannot (Linux before 5.14, mappings of devices) the write faults them in by itself
+static void populate(void* p, size_t bytes) {
+  if (!p || !bytes) return;
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p & ~(page - 1);
+  (void)madvise((void*)a, (((uintptr_t)p + bytes + page - 1) & ~(page - 1)) - a, MADV_POPULATE_WRITE);
+}
+
+// The caller's planes of a pair, while the GPU works on it: a program that allocates its results for each call gets as many
+// fresh pages as its allocator wills, and their faults held up the copies at a call's end. Five uneven pairs of 0.13 to
+// 0.79 Mpx, ms per call without and with it: 36.5 -> 29.0 with the C library's defaults, 41.4 -> 31.3 where every plane is
+// mapped anew, 29.3 -> 28.7 where none is.
+static void populate_out(const ofc_pair_out& o, size_t N) {
+  float* const f[10] = {o.ux, o.uy, o.conf, o.exx, o.eyy, o.exy, o.gmax, o.vol, o.raw_ux, o.raw_uy};
+  for (float* p : f) populate(p, N * 4);
+  populate(o.valid, N);
+}
+
 static void download_pair(Lane& L, const ofc_pair_out& d, ofc_pair_out* h, size_t N) {
   cudaStream_t st = L.stream;
   float* const* dsrc[10] = {&d.ux, &d.uy, &d.conf, &d.exx, &d.eyy, &d.exy, &d.gmax, &d.vol, &d.raw_ux, &d.raw_uy};
@@ -2248,6 +2272,7 @@ int ofc_track_pairs(ofc_engine* e, const ofc_pair_in* pairs, size_t n, const ofc
       uint8_t* hvalid = A.pinned<uint8_t>("batch_hvalid", N);
       OFC_CUDA(cudaMemcpyAsync(hout, d.ux, 10 * N * 4, cudaMemcpyDeviceToHost, A.stream));
       OFC_CUDA(cudaMemcpyAsync(hvalid, d.valid, N, cudaMemcpyDeviceToHost, A.stream));
+      populate_out(outs[i], N);
       OFC_CUDA(cudaStreamSynchronize(A.stream));
       ofc_pair_out o{};
       float** f[10] = {&o.ux, &o.uy, &o.conf, &o.exx, &o.eyy, &o.exy, &o.gmax, &o.vol, &o.raw_ux, &o.raw_uy};
@@ -2306,6 +2331,7 @@ int ofc_track_pairs(ofc_engine* e, const ofc_pair_in* pairs, size_t n, const ofc
       Lane& A = *L.aux[j];
       const size_t i = (size_t)busy[j], N = pairs[i].w * pairs[i].h;
       busy[j] = -1;
+      populate_out(outs[i], N);
       OFC_CUDA(cudaStreamSynchronize(A.stream));
       float* hout = A.pinned<float>("batch_hout", 10 * N);
       ofc_pair_out o{};
@@ -3222,6 +3248,8 @@ int ofc_test_local_solve(ofc_engine* e, const double* sums, const double* ux, co
     OFC_CUDA(cudaStreamSynchronize(L.stream));
   });
 }
+
+void ofc_test_populate(void* p, size_t bytes) { populate(p, bytes); }
 
 int ofc_test_median(ofc_engine* e, const double* v, size_t n, double* median, char* err, size_t errlen) {
   return guarded(e, err, errlen, [&](Lane& L) {

@@ -226,6 +226,7 @@ TEST_SIGNATURES = {
                              + [c_double_p] * 5 + [_E, _S]),
     "ofc_test_median": (ctypes.c_int, [_P, c_double_p, _S, c_double_p, _E, _S]),
     "ofc_test_median_reset": (ctypes.c_int, [_P, c_double_p, _S, _S, c_u8_p, c_double_p, c_double_p, c_double_p, _E, _S]),
+    "ofc_test_populate": (None, [_P, _S]),
     "ofc_test_large_components": (ctypes.c_int, [_P, c_u8_p, _S, _S, ctypes.c_double, c_u8_p, _E, _S]),
     "ofc_test_first_sums": (ctypes.c_int, [_P, c_float_p, c_float_p, _S, _S, c_double_p, c_double_p,
                                            ctypes.POINTER(OfcConfig), c_double_p, _E, _S]),

@@ -153,3 +153,29 @@ def test_no_launch_needs_the_whole_device():
     for f in files:
         text = open(f).read()
         assert "cudaLaunchCooperativeKernel" not in text and "cudaLaunchAttributeCooperative" not in text, f
+
+
+def test_populate(lib):
+    """The pages of a pair's planes are backed before they are written: whole pages of the range and no others, their
+    contents unchanged, ranges that start and end inside a page, null and empty ranges."""
+    import mmap
+    page, n = mmap.PAGESIZE, 12
+    libc = ctypes.CDLL(None, use_errno=True)
+    m = mmap.mmap(-1, n * page)
+    at = ctypes.addressof(ctypes.c_char.from_buffer(m))
+    if libc.madvise(ctypes.c_void_p(at), ctypes.c_size_t(page), 23) != 0:
+        pytest.skip("no MADV_POPULATE_WRITE")
+
+    def resident():
+        v = (ctypes.c_ubyte * n)()
+        assert libc.mincore(ctypes.c_void_p(at), ctypes.c_size_t(n * page), v) == 0
+        return [k for k in range(n) if v[k] & 1]
+
+    m[4 * page + 5] = 7
+    assert resident() == [0, 4]
+    lib.ofc_test_populate(None, 100)
+    lib.ofc_test_populate(at + 8 * page, 0)
+    assert resident() == [0, 4]
+    lib.ofc_test_populate(at + 3 * page + 40, 2 * page)
+    assert resident() == [0, 3, 4, 5]
+    assert m[4 * page + 5] == 7 and bytes(m[:]).count(0) == n * page - 1
