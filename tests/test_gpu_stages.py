@@ -387,6 +387,44 @@ def test_accumulate_ring_and_edges(T, shape, n_orient, scales):
     np.testing.assert_array_equal(s0, s1)
 
 
+@pytest.mark.parametrize("amp", [1e-30, 1e-24, 1e-18, 1e12, 1e18, 1e20, 1e22])
+def test_accumulate_extreme_amplitudes(T, amp):
+    """The accumulate's packed phase differences at response magnitudes beyond its fast quotient's range (products of two
+    responses below 1e-30 and above 1e30, infinite and NaN ones) against the TMA-staged kernel's unpacked arithmetic: bit
+    for bit but for the rounding of a quotient, at most one unit of the last place of a float32 angle (2.4e-7 of pi) in the
+    sums that hold it. Finite, infinite and NaN sums in the same places."""
+    rng = np.random.default_rng(11)
+    h, w = 67, 70
+    a, b = rng.random((h, w)), rng.random((h, w))
+    ux, uy = rng.normal(size=(2, h, w))
+    cfg = Config(n_orient=4, scales=(0.6,))
+    s0, _ = T.accumulate(a * amp, b * amp, ux, uy, mode=0, cfg=cfg)
+    s1, t1 = T.accumulate(a * amp, b * amp, ux, uy, mode=1, cfg=cfg)
+    assert t1 == 0
+    for i in (0, 1, 2, 6):  # no phase difference in these
+        np.testing.assert_array_equal(s0[i], s1[i])
+    for i in (3, 4, 5):
+        np.testing.assert_array_equal(np.isnan(s0[i]), np.isnan(s1[i]))
+        np.testing.assert_array_equal(np.isinf(s0[i]), np.isinf(s1[i]))
+        ok = np.isfinite(s1[i])
+        if ok.any():
+            np.testing.assert_allclose(s0[i][ok], s1[i][ok], rtol=1e-6, atol=1e-6 * np.abs(s1[i][ok]).max())
+
+
+def test_atan2_phase_exact_quotients(T):
+    """Magnitudes outside the fast quotient's range take the rounded quotient: arguments whose quotient is a power of two
+    give one angle, whatever their common factor (2^-120 to 2^-101 and 2^101 to 2^126, subnormal ones among them)."""
+    rng = np.random.default_rng(12)
+    m = rng.uniform(1, 2, 4000).astype(np.float32)
+    for lo, hi in ((-120, -101), (-140, -127), (101, 126)):
+        s = np.ldexp(m, rng.integers(lo, hi, m.size)).astype(np.float32)
+        for k in (0, 1, 3):
+            y, x = s, np.ldexp(s, -k).astype(np.float32)
+            same = np.ldexp(x.astype(np.float64), k) == y  # no bits lost to a subnormal
+            got = T.atan2(y[same], x[same])[0]
+            assert same.sum() > 100 and np.unique(got).size == 1, (lo, k)
+
+
 def test_atan2_phase(T):
     """The accumulate's float32 atan2 (common.cuh, a polynomial fit of atan on [0, 1]) within 5e-7 rad of the exact
     angle of its float32 arguments over 20 decades of magnitude and every direction, like CUDA's atan2f there; signed
