@@ -210,17 +210,27 @@ FftPlan fft_make_plan(int L, int variant) {
   return pl;
 }
 
+// W[t] = exp(-2 pi i t / L), t < L, rounded from float64
+static std::vector<float2> fft_twiddles(int L) {
+  std::vector<float2> t(L);
+  for (int i = 0; i < L; i++) {
+    double a = -2.0 * PI * (double)i / (double)L;
+    t[i] = make_float2((float)std::cos(a), (float)std::sin(a));
+  }
+  return t;
+}
+
 std::vector<float2> fft_tables(const FftPlan& pl) {
   const int SL = fft_work_len(pl);
   const std::vector<float2> tw = fft_twiddles(SL);
-  std::vector<float2> out = tw;
+  std::vector<float2> out;
   for (int i = 0; i < pl.nst; i++) {
     const int m = SL / (pl.p[i] * pl.s[i]);
     for (int k = 1; k < pl.p[i]; k++)
       for (int q = 0; q < m; q++) out.push_back(tw[(size_t)k * q * pl.s[i]]);
   }
-  const size_t n = out.size() - SL;  // the inverse transform's conjugates
-  for (size_t i = 0; i < n; i++) out.push_back(make_float2(out[SL + i].x, -out[SL + i].y));
+  const size_t n = out.size();  // the inverse transform's conjugates
+  for (size_t i = 0; i < n; i++) out.push_back(make_float2(out[i].x, -out[i].y));
   if (pl.M) {
     const std::vector<float2> bt = fft_bluestein_tables(pl.L, pl.M);
     out.insert(out.end(), bt.begin(), bt.end());
@@ -230,23 +240,13 @@ std::vector<float2> fft_tables(const FftPlan& pl) {
 
 void fft_bind(FftPlan& pl, const float2* d) {
   const int SL = fft_work_len(pl);
-  pl.tw = d;
-  pl.stw = d + SL;
+  pl.stw = d;
   const int last = pl.nst - 1;
   pl.nstw = pl.so[last] + (pl.p[last] - 1) * (SL / (pl.p[last] * pl.s[last]));
   if (pl.M) {
     pl.chirp = pl.stw + 2 * pl.nstw;
     pl.filt = pl.chirp + pl.L;
   }
-}
-
-std::vector<float2> fft_twiddles(int L) {
-  std::vector<float2> t(L);
-  for (int i = 0; i < L; i++) {
-    double a = -2.0 * PI * (double)i / (double)L;
-    t[i] = make_float2((float)std::cos(a), (float)std::sin(a));
-  }
-  return t;
 }
 
 // Threads of a block of a runtime plan that holds `smem` bytes: the count whose blocks finish most lines per time on an SM.
@@ -791,16 +791,16 @@ __device__ __forceinline__ bool fft_stage(const float2* A, float2* B, const FftP
   return osh;
 }
 
-// the plan's stages on their length SL (L, or Bluestein's M): the first reads `first` through IN, the last writes dst
-// through OUT, those between alternate between b and a (all unpadded at the ends). dst may be `first` or a with an odd
-// number of stages, b with an even one; a null dst takes that one, which is returned.
+// the plan's stages on their length SL (L, or Bluestein's M): the first reads `first` (a or neither buffer) through IN and
+// writes b, the next ones a, b, ... in turn, the last writes through OUT (first and result unpadded). The result goes to
+// dst, which is neither a nor b (it may be `first`: only the first of two or more stages reads that), or for a null dst to
+// the buffer that the last stage does not read; returned is where it is.
 template <int LC, int IN, int OUT>
 __device__ __forceinline__ float2* fft_stages(const float2* first, float2* a, float2* b, float2* dst, const FftPlan& pl,
                                               int SL, bool inv, const StageEx& ex) {
-  if (!dst) dst = pl.nst & 1 ? (pl.nst == 1 ? b : a) : a;
-  if (pl.nst == 1) {
-    fft_stage<LC, IN, OUT_PLAIN>(first, dst, pl, 0, SL, inv, false, ex);
-    return dst;
+  if (pl.nst == 1) {  // a line of one radix (the testing entry's: a padded line has two stages at least)
+    fft_stage<LC, IN, OUT_PLAIN>(first, b, pl, 0, SL, inv, false, ex);
+    return b;
   }
   bool ish = fft_stage<LC, IN, OUT_PLAIN>(first, b, pl, 0, SL, inv, false, ex);
   float2 *x = b, *y = a;
@@ -810,10 +810,13 @@ __device__ __forceinline__ float2* fft_stages(const float2* first, float2* a, fl
     x = y;
     y = t;
   }
-  if (dst == x) dst = y;
-  fft_stage<LC, IN_PLAIN, OUT>(x, dst, pl, pl.nst - 1, SL, inv, ish, ex);
-  return dst;
+  float2* to = dst ? dst : y;
+  fft_stage<LC, IN_PLAIN, OUT>(x, to, pl, pl.nst - 1, SL, inv, ish, ex);
+  return to;
 }
+// A line of one stage has no place for OUT and a dst. The lengths that have one are the radices, at most 31; a padded line
+// and a Bluestein inner length (at least 2 * 37 - 1) are longer.
+static_assert(2 * PAD + 1 > 31, "a padded line has two stages at least");
 
 // The 16 inner lengths that fft_work_length gives most of the 1316 lengths from 160 to 2048 with a prime factor above 31
 // (the 16th serves 26 of them, all together 69 %; a further length costs 13 s of compile time and serves under 2 %).

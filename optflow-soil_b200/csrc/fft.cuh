@@ -20,15 +20,16 @@ constexpr int FFT_TMAX = 512;  // threads per block at most
 constexpr int RT_T = 768;      // the same of the runtime plans' kernels (80 registers)
 
 // A 1-D plan of length L: mixed-radix Stockham stages (radix p[i], stride s[i] = product of the radices
-// before it) and the twiddle table W[t] = exp(-2 pi i t / L), t < L, rounded from float64. Stage i's twiddles lie together
-// as its butterflies read them, stw[so[i] + (k - 1) m + q] = W[k q s[i]] (m = L / (p[i] s[i]), k = 1 .. p[i] - 1, q < m):
-// neighbouring threads (consecutive q) read neighbouring values, where W itself is read at a stride of k s[i]; the nstw
-// values are followed by their conjugates (the inverse transform's). inner: M where its stages are in the default order
-// (the transforms of the common inner lengths are compiled for that order), else 0.
+// before it). With W[t] = exp(-2 pi i t / L), rounded from float64, stage i's twiddles lie together as its butterflies read
+// them, stw[so[i] + (k - 1) m + q] = W[k q s[i]] (m = L / (p[i] s[i]), k = 1 .. p[i] - 1, q < m): neighbouring threads
+// (consecutive q) read neighbouring values, where a table of W would be read at a stride of k s[i]; the nstw values are
+// followed by their conjugates (the inverse transform's). inner: M where its stages are in the default order (the
+// transforms of the common inner lengths are compiled for that order), else 0.
 // A length with a prime factor above 31 is transformed by Bluestein's chirp z-transform (as the reference's Metal
 // FFT does, rust/crates/optflow-gpu/src/fft.rs:1-3): M > 0 is then the inner length (a length >= 2L - 1 of
-// the radices with butterflies, of fewest stages: fft_work_length), the stages and tw are those of length M, chirp[n] = exp(-i pi n^2 / L) for n < L, and filt is the
-// length-M transform of the conjugate chirp (wrapped: index m and M - m for m < L) times 1 / M.
+// the radices with butterflies, of fewest stages: fft_work_length), the stages and stw are those of length M,
+// chirp[n] = exp(-i pi n^2 / L) for n < L, and filt is the length-M transform of the conjugate chirp (wrapped: index m and
+// M - m for m < L) times 1 / M.
 struct FftPlan {
   int L = 0;
   int nst = 0;
@@ -36,7 +37,6 @@ struct FftPlan {
   int s[FFT_MAXST] = {};
   unsigned magic[FFT_MAXST] = {};
   int so[FFT_MAXST] = {};
-  const float2* tw = nullptr;
   const float2* stw = nullptr;
   int nstw = 0;
   int inner = 0;
@@ -63,9 +63,8 @@ FftPlan fft_make_plan(int L, int variant);
 // engine has already built keep theirs
 void fft_set_plan_variant(int L, int variant);
 int fft_plan_variant(int L);
-std::vector<float2> fft_twiddles(int L);
 std::vector<float2> fft_bluestein_tables(int L, int M);
-// every table of a plan in one vector (twiddles, stage twiddles and, for Bluestein, the chirp and the filter), and the
+// every table of a plan in one vector (the stages' twiddles and, for Bluestein, the chirp and the filter), and the
 // binding of the plan to a device copy of it
 std::vector<float2> fft_tables(const FftPlan& pl);
 void fft_bind(FftPlan& pl, const float2* d);

@@ -24,6 +24,17 @@ def T():
 BLUESTEIN = [37, 164, 106, 604, 191, 1021, 1999]
 
 
+@pytest.mark.parametrize("L", [2, 3, 4, 5, 7, 8, 11, 13, 17, 19, 23, 29, 31])
+def test_fft_lines_one_stage(T, L):
+    """Lines of one radix, a transform whose first stage is its last: within the bound of test_fft_lines_runtime_plans."""
+    rng = np.random.default_rng(L)
+    a = (rng.standard_normal((5, L)) + 1j * rng.standard_normal((5, L))).astype(np.complex64)
+    for inv in (False, True):
+        got = T.fft_lines(a, inverse=inv)
+        ref = np.fft.ifft(a.astype(np.complex128), axis=1) * L if inv else np.fft.fft(a.astype(np.complex128), axis=1)
+        assert np.abs(got - ref).max() < 2e-6 * np.abs(ref).max(), inv
+
+
 @pytest.mark.parametrize("L,bound", [(144, 2e-6), (441, 2e-6), (650, 2e-6), (975, 2e-6), (1539, 2e-6), (2023, 2e-6),
                                       (2048, 2e-6), (253, 2e-6), (841, 2e-6), (899, 2e-6), (1564, 2e-6), (1922, 2e-6), (397, 1e-5), (433, 1e-5), (917, 1e-5), (1109, 1e-5),
                                       (1431, 1e-5), (1822, 1e-5)])
