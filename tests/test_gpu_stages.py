@@ -398,6 +398,64 @@ def test_accumulate_ring_and_edges(T, shape, n_orient, scales):
     np.testing.assert_array_equal(s0, s1)
 
 
+def test_accumulate_ring_cases_are_two_kernels(T):
+    """The two modes that test_accumulate_ring_and_edges compares are two kernels where there are two filters or more; one
+    filter has the gather kernel alone (its second slot of the ring is never filled), which test_accumulate_one_filter
+    checks."""
+    from optflow_b200.api import default_engine
+    from optflow_b200.measure import Profile
+    rng = np.random.default_rng(3)
+    for shape, n_orient, scales, staged in (((64, 65), 1, (1.0,), False), ((67, 131), 3, (0.6,), True),
+                                            ((130, 97), 5, (0.6,), True), ((70, 64), 4, (0.6, 1.0, 1.6), True)):
+        a, b = rng.random(shape), rng.random(shape)
+        u = np.zeros(shape)
+        prof = Profile(default_engine())
+        prof.start()
+        T.accumulate(a, b, u, u, mode=1, cfg=Config(n_orient=n_orient, scales=scales))
+        assert ("k_accumulate_tma" in prof.read()) == staged, shape
+
+
+@pytest.mark.parametrize("shape", [(64, 65), (67, 131)])
+def test_accumulate_one_filter(T, oracle, shape):
+    """The accumulate of a single filter (the second slot of its ring is never filled, the packed arithmetic's second half
+    works on whatever is there) against the oracle's float64 sums, positions beyond the padded plane included. Tolerance,
+    from the stages' (test_responses, test_reference_phase): responses within 1e-4 of their largest |r|, the phase gradient
+    within 1e-3 rad/px, where |r1| and |r2| exceed 5 % of it. So the weight |r1| |r2| within e_w = 2 * 1e-4 / 0.05 relative,
+    the phase difference within the same of 1 rad, c within e_c = e_w + 1e-3 (|u| + |v|), and the sums by the product rule.
+    Pixels whose phase difference may wrap (within 0.1 of pi) are left out."""
+    rng = np.random.default_rng(shape[1])
+    h, w = shape
+    from scipy.ndimage import gaussian_filter
+    a = gaussian_filter(rng.random((h, w)), 1.0).astype(np.float32)
+    b = np.roll(a, (1, 2), axis=(0, 1))
+    yy, xx = np.mgrid[0:h, 0:w].astype(np.float64)
+    ux, uy = 2 + np.sin(xx / 17.0), 1 + 0.5 * np.cos(yy / 23.0)
+    ux[:, :3] -= 70.0
+    uy[-3:] += 70.0
+    cfg = Config(n_orient=1, scales=(1.0,))
+    got, _ = T.accumulate(a, b, ux, uy, mode=0, cfg=cfg)
+    want = oracle.first_sums(a, b, ux, uy, cfg)
+    r, gx, gy, _ = oracle.reference_phase(a, cfg)[0]
+    wk = want[6]
+    r1 = np.abs(r)
+    r2 = wk / r1
+    c = np.where(np.abs(gx) > np.abs(gy), want[3] / (wk * gx), want[4] / (wk * gy))
+    ok = (r1 > 0.05 * r1.max()) & (r2 > 0.05 * r1.max()) & (np.abs(c - gx * ux - gy * uy) < np.pi - 0.1)
+    assert ok.mean() > 0.5
+    ew, eg = 2 * 1e-4 / 0.05, 1e-3
+    ec = ew + eg * (np.abs(ux) + np.abs(uy))
+    ax, ay, ac = np.abs(gx), np.abs(gy), np.abs(c)
+
+    def bound(p, ep, q, eq):  # of wk p q
+        return wk * ((1 + ew) * (p + ep) * (q + eq) - p * q)
+
+    bounds = [bound(ax, eg, ax, eg), bound(ax, eg, ay, eg), bound(ay, eg, ay, eg), bound(ax, eg, ac, ec),
+              bound(ay, eg, ac, ec), bound(ac, ec, ac, ec), wk * ew]
+    for i in range(7):
+        assert np.isfinite(got[i]).all()
+        assert (np.abs(got[i] - want[i]) <= bounds[i])[ok].all(), i
+
+
 @pytest.mark.parametrize("amp", [1e-30, 1e-24, 1e-18, 1e12, 1e18, 1e20, 1e22])
 def test_accumulate_extreme_amplitudes(T, amp):
     """The accumulate's packed phase differences at response magnitudes beyond its fast quotient's range (products of two
