@@ -31,6 +31,14 @@ struct Error : std::runtime_error {
                                              " at " + __FILE__ + ":" + std::to_string(__LINE__)); \
   } while (0)
 
+// A host-to-device copy that has ended on return. cudaMemcpy of pageable memory returns once the data are staged, before
+// they are all on the device, and work on the lanes' streams (which do not wait for the default stream) could read what was
+// there before.
+inline void upload_now(void* dst, const void* src, size_t bytes) {
+  OFC_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
+  OFC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+}
+
 // kernel launch with error check, the engine's launch counter and, in profile mode, CUDA events around the
 // launches whose kernel name matches the profile filter (the reference's per-kernel GPU timing,
 // OPTFLOW_GPU_KERNELS, rust/README.md:157-159)

@@ -326,7 +326,7 @@ struct Lane {
       b.reset(new DevBuf());
       OFC_CUDA(cudaMalloc(&b->p, std::max<size_t>(count * sizeof(T), 256)));
       b->bytes = count * sizeof(T);
-      OFC_CUDA(cudaMemcpy(b->p, host, count * sizeof(T), cudaMemcpyHostToDevice));
+      upload_now(b->p, host, count * sizeof(T));
     }
     return (const T*)b->p;
   }
@@ -359,7 +359,7 @@ struct Lane {
     size_t b32 = tw.size() * sizeof(float2);
     OFC_CUDA(cudaMalloc(&b->p, b32));
     b->bytes = b32;
-    OFC_CUDA(cudaMemcpy(b->p, tw.data(), b32, cudaMemcpyHostToDevice));
+    upload_now(b->p, tw.data(), b32);
     fft_bind(pl, (const float2*)b->p);
     auto& slot = plans[L];
     slot.first = pl;
@@ -3555,7 +3555,7 @@ int ofc_set_coarse_net(ofc_engine* e, const float* params, size_t n, int tile, d
       P->max_low = max_low_share;
       OFC_CUDA(cudaMalloc(&P->params, cnt * sizeof(float)));
       OFC_CUDA(cudaMalloc(&P->w16, cnt * sizeof(uint16_t)));
-      OFC_CUDA(cudaMemcpy(P->params, params, cnt * sizeof(float), cudaMemcpyHostToDevice));
+      upload_now(P->params, params, cnt * sizeof(float));
       net::Workspace ws{[](const std::string&, size_t) -> void* { return nullptr; }, e->lanes[0]->stream};
       net::to_bf16(ws, P->params, P->w16);
       OFC_CUDA(cudaStreamSynchronize(e->lanes[0]->stream));

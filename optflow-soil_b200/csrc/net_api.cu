@@ -106,6 +106,7 @@ ofc_net* ofc_net_create(int device, char* err, size_t errlen) {
     OFC_CUDA(cudaMemset(n->m, 0, P * 4));
     OFC_CUDA(cudaMemset(n->v, 0, P * 4));
     OFC_CUDA(cudaMemset(n->w16, 0, P * 2));
+    OFC_CUDA(cudaDeviceSynchronize());  // before any stream's first use
   });
   if (st != OFC_OK) {
     delete n;
@@ -126,7 +127,7 @@ int ofc_net_set_params(ofc_net* n, const float* params, size_t cnt, char* err, s
     const size_t P = ofc::net::param_count();
     if (!params || cnt != P) throw ofc::Error(OFC_ERR_ARG, "expected " + std::to_string(P) + " parameters");
     OFC_CUDA(cudaDeviceSynchronize());
-    OFC_CUDA(cudaMemcpy(n->params, params, P * 4, cudaMemcpyHostToDevice));
+    ofc::upload_now(n->params, params, P * 4);
     OFC_CUDA(cudaMemset(n->m, 0, P * 4));
     OFC_CUDA(cudaMemset(n->v, 0, P * 4));
     n->step = 0;

@@ -155,6 +155,29 @@ def test_no_launch_needs_the_whole_device():
         assert "cudaLaunchCooperativeKernel" not in text and "cudaLaunchAttributeCooperative" not in text, f
 
 
+def test_tables_have_landed_before_their_first_use():
+    """cudaMemcpy of pageable host memory returns before the data are on the device, and streams made non-blocking do not
+    wait for it: such a copy to the device is made by upload_now alone, which waits, and a network's first state is waited
+    for."""
+    import glob
+    import os
+    import re
+    csrc = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "optflow-soil_b200", "csrc")
+    copies, waits = [], []
+    for f in sorted(glob.glob(os.path.join(csrc, "*.cu")) + glob.glob(os.path.join(csrc, "*.cuh"))):
+        text = open(f).read()
+        copies += [(os.path.basename(f), m.start()) for m in re.finditer(r"cudaMemcpy\([^;]*cudaMemcpyHostToDevice", text)]
+        for m in re.finditer(r"cudaMemset\([^;]*;", text):  # the next call that waits, before the function ends
+            end = text.index("\n}", m.end())
+            waits.append("cudaDeviceSynchronize" in text[m.end():end])
+    assert [c[0] for c in copies] == ["common.cuh"]
+    common = open(os.path.join(csrc, "common.cuh")).read()
+    body = common[common.index("inline void upload_now"):]
+    body = body[:body.index("\n}")]
+    assert body.index("cudaMemcpy(") < body.index("cudaStreamSynchronize(cudaStreamLegacy)")
+    assert waits and all(waits)
+
+
 def test_populate(lib):
     """The pages of a pair's planes are backed before they are written: whole pages of the range and no others, their
     contents unchanged, ranges that start and end inside a page, null and empty ranges."""

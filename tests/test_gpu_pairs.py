@@ -54,3 +54,27 @@ def test_track_pairs_errors():
         track_pairs([items[0], (items[0][0][:40, :40], items[0][1][:40, :40])], Config())
     with pytest.raises(ValueError, match="ROI mask shape"):
         track_pairs([(items[0][0], items[0][1], np.ones((3, 3), bool))], Config())
+
+
+def test_first_call_equals_repeats():
+    """The first call of an engine at a size (it uploads the tables of that size: twiddles, filters, taps, matching windows)
+    gives the bits of the calls after it, on the caller's lane and on the workers of a batch. 16 engines each of two padded
+    sizes of one row pass on a runtime plan, 6 engines with a batch of uneven pairs."""
+    from optflow_b200 import Engine, testing
+    rng = np.random.default_rng(0)
+    for k in range(16):
+        eng = Engine(0)
+        for h, w in ((80, 695), (333, 191)):
+            img = rng.random((h, w)).astype(np.float32)
+            first = testing.responses(img, engine=eng)
+            np.testing.assert_array_equal(testing.responses(img, engine=eng), first, err_msg=f"{k}: {w} x {h}")
+        eng.close()
+    a, b = _synthetic_pair(256, 3)
+    items = [(a[:, :128], b[:, :128]), (a[:200, :256], b[:200, :256]), (a, b), (a[:96], b[:96])]
+    for k in range(6):
+        eng = Engine(0)
+        runs = [track_pairs(items, Config(), engine=eng) for _ in range(2)]
+        for i, (x, y) in enumerate(zip(*runs)):
+            for q in PLANES:
+                np.testing.assert_array_equal(getattr(x, q), getattr(y, q), err_msg=f"{k}: pair {i}: {q}")
+        eng.close()
