@@ -61,7 +61,7 @@ void prof_after(void* token, cudaStream_t st);
 // launch is prepared while that kernel drains, and its blocks wait in grid_dep_wait, which every kernel launched this way
 // calls before it touches memory, until that kernel has ended and its writes are visible. For the refinement's kernels,
 // some 150 dependent launches that small images wait for: 128^2 pairs 1.246 -> 1.216 ms, 256^2 1.588 -> 1.533 ms, 333 x
-// 191 2.198 -> 2.126 ms, from 512^2 up unchanged. No kernel releases its dependents early: their waiting blocks would
+// 191 2.198 -> 2.126 ms, from 512^2 up 0.2 to 1 %. No kernel releases its dependents early: their waiting blocks would
 // take its place on the SMs (2048^2: 30.3 -> 30.7 ms).
 #define OFC_LAUNCH_PDL(kernel, grid, block, smem, stream_, ...)                    \
   do {                                                                             \
@@ -128,10 +128,10 @@ __device__ __forceinline__ float atan2_ratio(float ax, float ay) {
   if (atan2_fast(mx)) return __fdividef(mn, mx);
   return mx > 0.f ? mn / mx : 0.f;
 }
-// the rounded quotient by the float64 reciprocal and two Newton steps, without the call that mn / mx takes: in the
-// accumulate's loop, where no usual value reaches it, a call costs 8 % of the kernel (0.513 against 0.472 ms at 2048^2) by
-// its register convention alone. The product is within 2^-51 of the quotient before its one rounding to float32. NaN where
-// both are
+// the rounded quotient by the float64 reciprocal and two Newton-Raphson steps (r + r (1 - d r)), without the call that
+// mn / mx takes: in the accumulate's loop, where no usual value reaches it, a call costs 8 % of the kernel (0.513 against
+// 0.472 ms at 2048^2) by its register convention alone. The product is within 2^-51 of the quotient before its one rounding
+// to float32. NaN where both are
 __device__ __forceinline__ float atan2_ratio_far(float mn, float mx) {
   const double d = (double)mx;
   double r;

@@ -1321,7 +1321,7 @@ __global__ void __launch_bounds__(FIXL > 0 ? 288 : FFT_TMAX, FIXL > 0 ? 3 : 2)
 // a block takes one node row. The two raw lines keep buffers of L values and receive
 // their own results; only the two scratch buffers have the work length (Bluestein's M is about 2 L). More blocks fit per
 // SM than with four buffers of M and a prefetch of the next row, and blocks of few threads (rt_threads) leave few
-// warps without a butterfly in the stages of large radices. Issue slots (55 %) and barriers bound it.
+// warps without a butterfly in the stages of large radices. Issue slots (59 %) and barriers bound it.
 template <int FIXL>
 __global__ void __launch_bounds__(RT_T, RT_MINB) k_fft_rows_inv_resp_rt(const float2* __restrict__ U, FftPlan plw, int ph, int F,
                                                                   float scale, float2* __restrict__ R) {

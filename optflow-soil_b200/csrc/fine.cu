@@ -359,19 +359,21 @@ void launch_warp_gather(const float* c2, int w2, int h2, const double* sx, const
 // pack; the field spline is stored interleaved (one 16-byte load per tap for both components); the responses are
 // stored in filter pairs, node-major, so one 16-byte load per tap serves two filters (96 tap loads per pixel at F = 12
 // instead of 192).
-// What bounds it is the latency and the issue slots of about 2200 instructions per pixel (DRAM at a third). Measured at
-// 2048^2, F = 12, against 0.572 ms per launch before (the same sums bit for bit):
-//   - the reference pack comes by asynchronous copies into a ring of two filter pairs instead of all F filters at once:
-//     32 KB of shared memory per SM instead of 192 KB leave L1 room for the taps of the resident blocks (0.573 ->
-//     0.534 ms with the changes below; a ring of three pairs 0.482 against 0.478 ms);
-//   - the taps' float32 sums and the two filters' atan polynomials run in packed instructions (fma.rn.f32x2: two
-//     values per issue slot, each rounded as by fmaf), the quotient of atan2 needs no branch, and the positions whose
-//     taps would mirror or clamp (at the plane's border) go out of line, so that the rest tests its range once;
-//   - 32 x 4 pixels per block, 7 blocks per SM at 72 registers: 0.478 ms (8 blocks at 64 registers 0.503, 6 at 80
-//     0.507, 32 x 8 pixels at 4 blocks 0.503).
+// What bounds it is L1: the response taps, their prefetches and the ring keep it at 90 % of its throughput (DRAM at 43 %,
+// issue at 50 %). 0.470 ms per launch in a 2048^2 pair, F = 12 (0.572 before the three steps below, the same sums bit for
+// bit). The forms, one built beside the other, by python -m optflow_b200.measure accumulate (2048^2, the kernel repeated on
+// one input): 0.433 ms as it is, and
+//   - the reference pack by asynchronous copies into a ring of two filter pairs: a ring of three pairs 0.452, all of the
+//     pairs staged at once 0.484 (24 KB per block instead of 8 leave L1 less room for the taps of the resident blocks);
+//   - the taps' float32 sums and the two filters' atan polynomials in packed instructions (fma.rn.f32x2: two values per
+//     issue slot, each rounded as by fmaf), the quotient of atan2 without a call, and the positions whose taps would mirror
+//     or clamp (at the plane's border) out of line, so that the rest tests its range once;
+//   - 32 x 4 pixels per block, 7 blocks per SM at 72 registers: 8 blocks at 64 registers 0.457, 6 at 80 0.459, 32 x 8 pixels
+//     at 4 blocks 0.456;
+//   - the next pair's tap rows prefetched into L1: 0.479 without.
 // Slower, and not kept: two pixels of a column per thread sharing their tap rows (L1 wavefronts fall by a third, but
-// 128 registers leave 16 warps per SM: 0.66 ms); the fixed point in a kernel of its own (0.122 + 0.424 ms: its loads no
-// longer overlap the sums' arithmetic).
+// 128 registers leave 16 warps per SM: 0.66 ms in the pair); the fixed point in a kernel of its own (0.122 + 0.424 ms: its
+// loads no longer overlap the sums' arithmetic).
 constexpr int ACC_BX = 32, ACC_BY = 4, ACC_T = ACC_BX * ACC_BY, ACC_MINB = 7;
 constexpr int ACC_ST = 2;       // filter pairs in the ring of the reference pack
 constexpr int ACC_MAXF = 56;    // the filters an earlier form held in shared memory at once; more stay refused
@@ -1140,8 +1142,10 @@ void launch_moments_solve(const double* sums, const double* ux, const double* uy
 // Small images are bound by the launches' latency: up to MED_CLUSTER_N energies one cluster of 8 blocks does it all
 // (k_median_cluster; 300 x 300 pairs 2228 us against 2252 with a launch per step, 360 x 360 3623 against 3593). Beyond, a
 // launch per step over the whole chip, whose last block to finish picks (k_median_range, k_median_hist, k_median_select,
-// k_median_reset). With energies over 50 octaves (60 % of a frame dark) the candidates are many and one block's select of
-// them takes 10 us of a launch more (2048^2: 45.7 ms per pair, as before).
+// k_median_reset). us per launch of a forced median at 2048^2: range 14, histogram 15 to 19, select 21. Where the energies'
+// range is stretched the part is wide, the candidates many, and the last block alone goes through them: select 97 with ties
+// of three values, 395 with one zero energy among ordinary ones; a frame whose dark 60 % span five octaves 21. A pair of
+// 2048^2 pixels, 60 % of them dark, takes 45.7 ms with it as it did with the cooperative form.
 constexpr size_t MED_CLUSTER_N = 98304;
 __device__ __forceinline__ unsigned long long okey(double v) {  // order-preserving key of a double
   unsigned long long u = (unsigned long long)__double_as_longlong(v);
