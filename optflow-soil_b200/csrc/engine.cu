@@ -321,14 +321,15 @@ struct Lane {
   std::unordered_map<std::string, std::unique_ptr<DevBuf>> consts;
   template <class T>
   const T* cached(const std::string& key, const T* host, size_t count) {
-    auto& b = consts[key];
-    if (!b) {
-      b.reset(new DevBuf());
+    auto it = consts.find(key);
+    if (it == consts.end()) {  // kept once it is whole: a call that fails here leaves no table without data behind
+      std::unique_ptr<DevBuf> b(new DevBuf());
       OFC_CUDA(cudaMalloc(&b->p, std::max<size_t>(count * sizeof(T), 256)));
       b->bytes = count * sizeof(T);
       upload_now(b->p, host, count * sizeof(T));
+      it = consts.emplace(key, std::move(b)).first;
     }
-    return (const T*)b->p;
+    return (const T*)it->second->p;
   }
   bool has_const(const std::string& key) const { return consts.count(key) != 0; }
 
@@ -500,7 +501,7 @@ GaborTables upload_gabor(Lane& L, int ph, int pw, const ofc_config& c) {
   const std::string key = "gabor:" + std::to_string(ph) + "x" + std::to_string(pw) + ":" + cfg_key(c);
   const double* d64;
   const float* d32;
-  if (L.has_const(key)) {
+  if (L.has_const(key) && L.has_const(key + ":f32")) {
     d64 = L.cached<double>(key, nullptr, 0);
     d32 = L.cached<float>(key + ":f32", nullptr, 0);
   } else {

@@ -178,6 +178,21 @@ def test_tables_have_landed_before_their_first_use():
     assert waits and all(waits)
 
 
+def test_a_failed_upload_leaves_no_table_behind():
+    """A lane keeps a table once it is allocated and uploaded: where either fails (no memory left), the next call starts over
+    and launches no kernel on a table without data. The filters' tables are two, and either may be the one that failed."""
+    import os
+    src = open(os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "optflow-soil_b200", "csrc", "engine.cu")).read()
+    body = src[src.index("const T* cached(const std::string& key"):]
+    body = body[:body.index("\n  }")]
+    assert body.index("cudaMalloc(") < body.index("upload_now(") < body.index("consts.emplace(") and "consts[" not in body
+    body = src[src.index("const FftPlan& plan(int L) {"):]
+    body = body[:body.index("\n  }")]
+    assert body.index("cudaMalloc(") < body.index("upload_now(") < body.index("plans[L]")
+    body = src[src.index("GaborTables upload_gabor("):]
+    assert 'has_const(key) && L.has_const(key + ":f32")' in body[:body.index("\n}")]
+
+
 def test_populate(lib):
     """The pages of a pair's planes are backed before they are written: whole pages of the range and no others, their
     contents unchanged, ranges that start and end inside a page, null and empty ranges."""
